@@ -204,18 +204,20 @@ int ct_curves_pitch(int32_t width, size_t* pitch_bytes);
 int ct_bm_census_process_curves(ct_handle* h, const ct_image* disp, const ct_curves* curves,
                                 const ct_image* left, const ct_image* right, ct_stream stream);
 
-/* Autotuner: times the kernel variants (4 or 8 disparities per warp) and
- * strip heights for this handle's (W, H, D, direction) on the given images,
- * keeps the fastest in the handle for later process calls. Synchronises
+/* Autotuner: times the CUDA-core kernel's variants (4 or 8 disparities per
+ * warp) and strip heights, and the tensor-core kernel, for this handle's (W, H,
+ * D, direction) on the given images, keeps the fastest in the handle for later
+ * process calls. Synchronises
  * `stream`. (No counterpart in the reference, whose launch shapes are
  * compile-time SConfig constants, BlockMatcherNCC.h:43-79.) */
 int ct_bm_census_autotune(ct_handle* h, const ct_image* left, const ct_image* right, ct_stream stream);
-/* The handle's current launch shape (strip height in rows, disparities per
- * warp); either pointer may be NULL. */
+/* The handle's current launch shape of the CUDA-core kernel (strip height in
+ * rows, disparities per warp); either pointer may be NULL. (The tensor-core
+ * kernel, which runs where it is the faster one, has one shape per size.) */
 int ct_bm_census_tuning(ct_handle* h, int32_t* strip_height, int32_t* disp_per_warp);
 /* Sets the launch shape (e.g. from a saved tuning table): strip_height with
- * strip_height + 4 a multiple of 5 (11..511), disp_per_warp 4 or 8. Results do
- * not depend on it. */
+ * strip_height + 4 a multiple of 5 (11..511), disp_per_warp 4 or 8, and selects
+ * the CUDA-core kernel. Results do not depend on it. */
 int ct_bm_census_set_tuning(ct_handle* h, int32_t strip_height, int32_t disp_per_warp);
 /* ct_bm_census_process_lr computes both directions in one matching pass by
  * default: the 5x5 Hamming cost of right pixel x_R at disparity e is the

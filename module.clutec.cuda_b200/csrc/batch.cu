@@ -112,7 +112,7 @@ __device__ void crosscheck_rows(const PairDev& P, int y0, int y1, int nt) {
             const int d = int(v) - 1, xo = x - d;
             if (xo >= 0 && xo < W) {
                 const bool inside = y >= cm::kAR && y < P.H - cm::kAR && xo >= cm::kAR && xo < W - cm::kAR;
-                const uint16_t vo = cm::rl_code<uint16_t>(__ldcg(P.rl_keys + (size_t)y * P.rl_pitch + xo), 0u, inside);
+                const uint16_t vo = cm::MinKeys{0u}.code<uint16_t>(__ldcg(P.rl_keys + (size_t)y * P.rl_pitch + xo), inside);
                 keep = abs(int(vo) - int(v)) <= P.tol;  // raw codes, CrossCheckDisparityMaps.cu:94
             }
         }

@@ -6,6 +6,7 @@
 #include "ct_internal.h"
 #include "ct_device.cuh"
 #include "census_match.cuh"
+#include "census_tc.cuh"
 #include "census_tile.cuh"
 
 namespace ct {
@@ -128,7 +129,8 @@ struct BmCensusHandle : ct_handle {
     uint32_t* keys = nullptr;      // ceil(D/64) planes of W*H merge keys
     uint32_t* counters = nullptr;  // one per (strip, column tile); 0 between calls
     uint32_t* rl_keys = nullptr;   // right-view keys of the fused pass, rows of cm::rl_pitch_words(W)
-    int rl_next_tag = cm::kRLTags - 1;  // tag of the next fused pass; < 0: reset the plane first
+    bool rl_max_keys = false;      // kind of the keys in the plane, and tags used since it was last set (next_tag)
+    int rl_tags_used = 0;
     int fuse_rl = 1;               // process_lr: right-to-left winners from the left-to-right pass
     uint16_t* tmp_lr = nullptr;    // U16 maps for process_lr when the caller wants only one
     uint16_t* tmp_rl = nullptr;
@@ -136,6 +138,10 @@ struct BmCensusHandle : ct_handle {
     CUtensorMap tm_lb, tm_rb, tm_lm, tm_rm;  // left/right as base (box 128) / match (box 192)
     int th = 36;   // strip height, chosen in configure or by the autotuner
     int dpw = 4;   // disparities per warp (kernel variant)
+    ctc::Shape tc{};   // tile shape and strip height of the tensor-core pass
+    int tc_rows = 0;
+    bool use_tc = false;        // left-to-right (and fused) passes on the tensor cores (tc_faster)
+    bool use_tc_right = false;  // and passes for the right view alone
     uint64_t* left_desc() const { return desc; }
     uint64_t* right_desc() const { return desc + (size_t)fmt.height * desc_pitch; }
 };
@@ -150,11 +156,11 @@ H* as(ct_handle* h, Kind k) {
     return (h && h->kind == k) ? static_cast<H*>(h) : nullptr;
 }
 
-// rl_tag >= 0: the left-to-right pass also bids for the right view into
-// h->rl_keys with that tag (the fused kernel).
+// rl_tag: the left-to-right pass also bids for the right view into h->rl_keys
+// with that tag (the fused kernel).
 int census_match_pass_maps(BmCensusHandle* h, int dir, const ct_image* disp, const CUtensorMap& tb,
                            const CUtensorMap& tm, cudaStream_t s, const ct_curves* curves = nullptr,
-                           int rl_tag = -1) {
+                           const uint32_t* rl_tag = nullptr) {
     using namespace cm;
     MatchArgs a{};
     a.W = h->fmt.width; a.H = h->fmt.height;
@@ -174,10 +180,10 @@ int census_match_pass_maps(BmCensusHandle* h, int dir, const ct_image* disp, con
         a.curve_pitch = curves->pitch_bytes / 4;
         a.curve_groups = (a.D + 3) / 4;
     }
-    if (rl_tag >= 0) {  // left-to-right pass bidding for the right view too
+    if (rl_tag) {  // left-to-right pass bidding for the right view too
         a.rl_keys = h->rl_keys;
         a.rl_pitch = rl_pitch_words(a.W);
-        a.rl_tag = uint32_t(rl_tag) << kRLTagShift;
+        a.rl_tag = *rl_tag;
     }
     const cudaError_t e = dir == 0 ? launch_census_match<0>(tb, tm, a, s, h->dpw)
                                    : launch_census_match<1>(tb, tm, a, s, h->dpw);
@@ -185,24 +191,31 @@ int census_match_pass_maps(BmCensusHandle* h, int dir, const ct_image* disp, con
     return CT_OK;
 }
 
-// process_lr in one matching pass: the left-to-right kernel decides both
-// directions' winners (the left map into lr, the right view's as tagged keys),
-// then one kernel writes the right-view map (disp_rl, when asked for) and the
-// cross-check of lr against the keys (disp_checked, when asked for).
-int census_process_fused(BmCensusHandle* h, const ct_image* lr, const ct_image* disp_rl,
-                         const ct_image* disp_checked, int tol, cudaStream_t s) {
+// Tag of the next pass that bids into the right-view keys. Min keys (the
+// CUDA-core pass) count their tags down, max keys (the tensor-core pass) up
+// from 1, so a call's bids beat what earlier calls left; the plane is set again
+// when every tag was used, or when the other kind was used before.
+int next_tag(BmCensusHandle* h, bool max_keys, cudaStream_t s, uint32_t* tag) {
+    using namespace cm;
+    if (h->rl_max_keys != max_keys || h->rl_tags_used >= kRLTags - 1) {
+        CT_CUDA_TRY(cudaMemsetAsync(h->rl_keys, max_keys ? 0 : 0xFF,
+                                    rl_pitch_words(h->fmt.width) * size_t(h->fmt.height) * 4, s));
+        h->rl_max_keys = max_keys;
+        h->rl_tags_used = 0;
+    }
+    const uint32_t n = uint32_t(h->rl_tags_used++);
+    *tag = (max_keys ? n + 1 : uint32_t(kRLTags - 1) - n) << kRLTagShift;
+    return CT_OK;
+}
+
+// Maps from the right-view keys of a pass: the right-view map (disp_rl) and the
+// cross-check of the left map lr (disp_checked), each when given.
+template <typename T, typename Keys>
+int launch_rl_check(BmCensusHandle* h, Keys how, const ct_image* lr, const ct_image* disp_rl,
+                    const ct_image* disp_checked, int tol, cudaStream_t s) {
     using namespace cm;
     const int W = h->fmt.width, H = h->fmt.height;
-    const size_t kpitch = rl_pitch_words(W);
-    if (h->rl_next_tag < 0) {  // every tag used since the plane was last set: set it again
-        CT_CUDA_TRY(cudaMemsetAsync(h->rl_keys, 0xFF, kpitch * H * 4, s));
-        h->rl_next_tag = kRLTags - 1;
-    }
-    const int tag_no = h->rl_next_tag--;
-    if (int rc = census_match_pass_maps(h, 0, lr, h->tm_lb, h->tm_rm, s, nullptr, tag_no)) return rc;
-    const uint32_t tag = uint32_t(tag_no) << kRLTagShift;
-    const int type = lr->type;
-    const int px = 16 / int(pix_size(type));
+    constexpr int px = 16 / int(sizeof(T));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((W + 128 * px - 1) / (128 * px), H);
     cfg.blockDim = dim3(128);
@@ -212,20 +225,79 @@ int census_process_fused(BmCensusHandle* h, const ct_image* lr, const ct_image* 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    void* rl_ptr = disp_rl ? disp_rl->ptr : nullptr;
-    const size_t rl_pb = disp_rl ? disp_rl->pitch_bytes : 0;
-    void* ck_ptr = disp_checked ? disp_checked->ptr : nullptr;
-    const size_t ck_pb = disp_checked ? disp_checked->pitch_bytes : 0;
-    if (type == CT_PIX_U8)
-        CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, rl_check_kernel<uint8_t>, h->rl_keys, kpitch, tag, W, H, int(kAR),
-                                       static_cast<uint8_t*>(rl_ptr), rl_pb, static_cast<const uint8_t*>(lr->ptr),
-                                       lr->pitch_bytes, static_cast<uint8_t*>(ck_ptr), ck_pb, tol));
-    else
-        CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, rl_check_kernel<uint16_t>, h->rl_keys, kpitch, tag, W, H, int(kAR),
-                                       static_cast<uint16_t*>(rl_ptr), rl_pb, static_cast<const uint16_t*>(lr->ptr),
-                                       lr->pitch_bytes, static_cast<uint16_t*>(ck_ptr), ck_pb, tol));
+    auto ptr = [](const ct_image* im) { return im ? static_cast<T*>(im->ptr) : nullptr; };
+    auto pitch = [](const ct_image* im) { return im ? im->pitch_bytes : size_t(0); };
+    CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, rl_check_kernel<T, Keys>, static_cast<const uint32_t*>(h->rl_keys),
+                                   rl_pitch_words(W), how, W, H, int(kAR), ptr(disp_rl), pitch(disp_rl),
+                                   static_cast<const T*>(ptr(lr)), pitch(lr), ptr(disp_checked),
+                                   pitch(disp_checked), tol));
     CT_LAUNCH_CHECK();
     return CT_OK;
+}
+
+template <typename Keys>
+int rl_check(BmCensusHandle* h, int type, Keys how, const ct_image* lr, const ct_image* disp_rl,
+             const ct_image* disp_checked, int tol, cudaStream_t s) {
+    return type == CT_PIX_U8 ? launch_rl_check<uint8_t>(h, how, lr, disp_rl, disp_checked, tol, s)
+                             : launch_rl_check<uint16_t>(h, how, lr, disp_rl, disp_checked, tol, s);
+}
+
+// process_lr in one matching pass: the left-to-right kernel decides both
+// directions' winners (the left map into lr, the right view's as tagged keys),
+// then one kernel writes the right-view map (disp_rl, when asked for) and the
+// cross-check of lr against the keys (disp_checked, when asked for).
+int census_process_fused(BmCensusHandle* h, const ct_image* lr, const ct_image* disp_rl,
+                         const ct_image* disp_checked, int tol, cudaStream_t s) {
+    uint32_t tag;
+    if (int rc = next_tag(h, false, s, &tag)) return rc;
+    if (int rc = census_match_pass_maps(h, 0, lr, h->tm_lb, h->tm_rm, s, nullptr, &tag)) return rc;
+    return rl_check(h, lr->type, cm::MinKeys{tag}, lr, disp_rl, disp_checked, tol, s);
+}
+
+// One pass on the tensor cores over the handle's row-major descriptors: the
+// left map (lr), the right-view map and the cross-check of lr, each when given
+// (lr is, with the cross-check).
+int census_process_tc(BmCensusHandle* h, const ct_image* lr, const ct_image* disp_rl, const ct_image* disp_checked,
+                      int tol, cudaStream_t s) {
+    const bool need_r = disp_rl || disp_checked;
+    uint32_t tag = 0;
+    if (need_r && lr) {
+        if (int rc = next_tag(h, true, s, &tag)) return rc;
+    } else if (need_r) {
+        // the right view alone: a plane set for this call only, so that the
+        // call can be captured and replayed as its CUDA-core pass can
+        CT_CUDA_TRY(cudaMemsetAsync(h->rl_keys, 0, cm::rl_pitch_words(h->fmt.width) * size_t(h->fmt.height) * 4, s));
+        h->rl_tags_used = cm::kRLTags;  // the next call sets it again
+        tag = 1u << cm::kRLTagShift;
+    }
+    ctc::Args a{};
+    a.W = h->fmt.width; a.H = h->fmt.height; a.D = h->par.disp_count;
+    a.dmin = h->par.disp_min;
+    a.mo = h->tc.mo; a.n = h->tc.n; a.th = h->tc_rows;
+    a.lstep = h->tc.lstep; a.rstep = h->tc.rstep;
+    a.left = h->left_desc(); a.right = h->right_desc();
+    a.pitch = h->desc_pitch;
+    if (lr) {
+        a.out = lr->ptr; a.out_pitch = lr->pitch_bytes; a.out_type = lr->type;
+    }
+    a.r_keys = need_r ? h->rl_keys : nullptr;
+    a.key_pitch = cm::rl_pitch_words(a.W);
+    a.tag = tag;
+    a.status = h->d_status;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(h->tc.tiles_x, (a.H + a.th - 1) / a.th);
+    cfg.blockDim = dim3(ctc::kNT);
+    cfg.dynamicSmemBytes = ctc::kSmemBytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];  // as launch_census_match
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, ctc::census_tc_kernel, a));
+    CT_LAUNCH_CHECK();
+    if (!need_r) return CT_OK;
+    return rl_check(h, (disp_rl ? disp_rl : disp_checked)->type, cm::MaxKeys{tag, a.dmin}, lr, disp_rl, disp_checked, tol, s);
 }
 
 int census_match_pass(BmCensusHandle* h, int dir, const ct_image* disp, cudaStream_t s,
@@ -234,8 +306,24 @@ int census_match_pass(BmCensusHandle* h, int dir, const ct_image* disp, cudaStre
                     : census_match_pass_maps(h, 1, disp, h->tm_rb, h->tm_lm, s, curves);
 }
 
-int census_both(BmCensusHandle* h, const ct_image* left, const ct_image* right, cudaStream_t s) {
-    return census::launch9x7_pair(left, right, h->left_desc(), h->right_desc(), h->desc_pitch, h->d_status, s, 1);
+// Where the tensor-core pass (census_tc.cuh) is the faster one, over whole calls
+// of 160x96 .. 2560x1440 pixels. It takes about as long for few disparities as
+// for 113 (128 left pixels a tile whatever the band), so the CUDA-core pass
+// wins below 48 on images that fill the GPU: at 1920x1080 checked maps take
+// 124 us against 111 (CUDA cores) for D = 32, 124 / 124 for 48, 123 / 136 for
+// 64, 138 / 263 for 128, 255 / 506 for 256. Small images are latency-bound and
+// its single launch without a merge wins at every D (640x480: 35 / 37 us at D
+// = 32, 37 / 68 at 128; 160x96: 21 / 29 at 64). The right view alone needs the
+// key plane set and read: from 65 disparities (1920x1080: 111 / 114 us at 64,
+// 113 / 194 at 96).
+bool tc_faster(int W, int H, int D, bool left) {
+    if (!left) return D > 64;
+    return D >= 48 || (long)W * H <= 400000;
+}
+
+int census_both(BmCensusHandle* h, const ct_image* left, const ct_image* right, cudaStream_t s, int planar = 1) {
+    return census::launch9x7_pair(left, right, h->left_desc(), h->right_desc(), h->desc_pitch, h->d_status, s,
+                                  planar);
 }
 
 }  // namespace
@@ -360,7 +448,14 @@ int ct_bm_census_configure(ct_handle* hh, int32_t device, const ct_format* fmt, 
     const size_t rl_bytes = cm::rl_pitch_words(W) * H * 4;
     if (cudaMalloc(&h->rl_keys, rl_bytes) != cudaSuccess) return fail(CT_ENOMEM, "right-view key scratch");
     CT_CUDA_TRY(cudaMemset(h->rl_keys, 0xFF, rl_bytes));
-    h->rl_next_tag = cm::kRLTags - 1;
+    h->rl_max_keys = false;
+    h->rl_tags_used = 0;
+    h->use_tc = tc_faster(W, H, p->disp_count, true);
+    h->use_tc_right = tc_faster(W, H, p->disp_count, false);
+    h->tc = ctc::pick_shape(W, p->disp_count);
+    h->tc_rows = ctc::pick_rows(H, h->tc.tiles_x, sm_count(device));
+    CT_CUDA_TRY(cudaFuncSetAttribute(ctc::census_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     ctc::kSmemBytes));
     h->fmt = *fmt;  // left_desc() / right_desc() below depend on the height
     h->th = cm::pick_strip_height(W, H, p->disp_count, sm_count(device));
     CT_CUDA_TRY(cm::prepare_census_match());
@@ -401,6 +496,11 @@ int ct_bm_census_process(ct_handle* hh, const ct_image* disp, const ct_image* le
     if (int rc = use_device(h->device)) return rc;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     h->last_stream = s;
+    if (h->par.left_to_right ? h->use_tc : h->use_tc_right) {
+        if (int rc = census_both(h, left, right, s, 0)) return rc;
+        return h->par.left_to_right ? census_process_tc(h, disp, nullptr, nullptr, 0, s)
+                                    : census_process_tc(h, nullptr, disp, nullptr, 0, s);
+    }
     if (int rc = census_both(h, left, right, s)) return rc;
     return census_match_pass(h, h->par.left_to_right ? 0 : 1, disp, s);
 }
@@ -453,14 +553,16 @@ int ct_bm_census_process_lr(ct_handle* hh, const ct_image* disp_lr, const ct_ima
     if (int rc = use_device(h->device)) return rc;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     h->last_stream = s;
-    if (int rc = census_both(h, left, right, s)) return rc;
+    const bool need_lr = disp_lr || disp_checked, need_rl = disp_rl || disp_checked;
+    const bool tc = need_lr ? h->use_tc && (!need_rl || h->fuse_rl) : h->use_tc_right;
+    if (int rc = census_both(h, left, right, s, tc ? 0 : 1)) return rc;
     const int W = h->fmt.width, H = h->fmt.height;
     ct_image tlr{h->tmp_lr, h->tmp_pitch, W, H, t, 0};
     ct_image trl{h->tmp_rl, h->tmp_pitch, W, H, t, 0};
     if (t == CT_PIX_U8) { tlr.pitch_bytes = trl.pitch_bytes = h->tmp_pitch; }
     const ct_image* lr = disp_lr ? disp_lr : &tlr;
+    if (tc) return census_process_tc(h, need_lr ? lr : nullptr, disp_rl, disp_checked, tol, s);
     const ct_image* rl = disp_rl ? disp_rl : &trl;
-    const bool need_lr = disp_lr || disp_checked, need_rl = disp_rl || disp_checked;
     if (need_lr && need_rl && h->fuse_rl)  // the same maps as two passes
         return census_process_fused(h, lr, disp_rl, disp_checked, tol, s);
     {
@@ -494,27 +596,39 @@ int ct_bm_census_autotune(ct_handle* hh, const ct_image* left, const ct_image* r
     float best_ms = 1e30f;
     int best_th = th0, best_dpw = 4;
     int rc = CT_OK;
+    // best of 3 timed passes after a warm-up
+    auto timed = [&](auto&& pass, float* best) -> int {
+        if (int r = pass()) return r;
+        *best = 1e30f;
+        for (int rep = 0; rep < 3; ++rep) {
+            cudaEventRecord(e0, s);
+            if (int r = pass()) return r;
+            cudaEventRecord(e1, s);
+            const cudaError_t e = cudaEventSynchronize(e1);
+            if (e != cudaSuccess) return fail(CT_ECUDA, "autotune timing failed: %s", cudaGetErrorString(e));
+            float ms = 0.f;
+            cudaEventElapsedTime(&ms, e0, e1);
+            *best = ms < *best ? ms : *best;
+        }
+        return CT_OK;
+    };
     for (int dpw : {4, 8}) {
         for (int th : ths) {
             if (th < 11 || (th + 2 * cm::kAR) % cm::kRB != 0) continue;
             h->dpw = dpw;
             h->th = th;
-            if ((rc = census_match_pass(h, dir, &out, s))) break;  // warm-up
-            float t = 1e30f;
-            for (int rep = 0; rep < 3 && rc == CT_OK; ++rep) {
-                cudaEventRecord(e0, s);
-                rc = census_match_pass(h, dir, &out, s);
-                cudaEventRecord(e1, s);
-                const cudaError_t e = cudaEventSynchronize(e1);
-                if (e != cudaSuccess) { rc = fail(CT_ECUDA, "autotune timing failed: %s", cudaGetErrorString(e)); break; }
-                float ms = 0.f;
-                cudaEventElapsedTime(&ms, e0, e1);
-                t = ms < t ? ms : t;
-            }
-            if (rc) break;
+            float t;
+            if ((rc = timed([&] { return census_match_pass(h, dir, &out, s); }, &t))) break;
             if (t < best_ms) { best_ms = t; best_th = th; best_dpw = dpw; }
         }
         if (rc) break;
+    }
+    // the tensor-core pass, on row-major descriptors
+    if (!rc && !(rc = census_both(h, left, right, s, 0))) {
+        float t;
+        rc = timed([&] { return dir == 0 ? census_process_tc(h, &out, nullptr, nullptr, 0, s)
+                                         : census_process_tc(h, nullptr, &out, nullptr, 0, s); }, &t);
+        if (!rc) (dir == 0 ? h->use_tc : h->use_tc_right) = t < best_ms;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -551,6 +665,7 @@ int ct_bm_census_set_tuning(ct_handle* hh, int32_t strip_height, int32_t disp_pe
     if (disp_per_warp != 4 && disp_per_warp != 8) return fail(CT_EINVAL, "disp_per_warp must be 4 or 8");
     h->th = strip_height;
     h->dpw = disp_per_warp;
+    h->use_tc = h->use_tc_right = false;  // the shape asked for is the CUDA-core kernel's
     return CT_OK;
 }
 

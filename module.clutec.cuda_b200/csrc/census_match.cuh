@@ -649,16 +649,33 @@ __global__ void __launch_bounds__(Var<DPW>::kNT, 1)
     run_tile<DIR, DPW, CURVE, RL>(&tmB, &tmM, a, t, sm, par);
 }
 
-// Map code of a right-view key of the fused pass (what store_disp writes
-// for it): a disparity iff the key carries this call's tag, a cost below
-// 2047 and the pixel is inside the border.
+// Map code of a disparity, or of none.
 template <typename T>
-__device__ __forceinline__ T rl_code(uint32_t key, uint32_t tag, bool inside) {
-    const bool ok = inside && (key & (0x1Fu << kRLTagShift)) == tag && ((key >> 16) & 0x7FFu) < 2047u;
-    const uint32_t d = key & 0xFFFFu;
+__device__ __forceinline__ T disp_code(bool ok, uint32_t d) {
     if constexpr (sizeof(T) == 1) return ok ? T(d) : T(0xFF);
     else return ok ? T(d + 1) : T(0xFFFF);
 }
+// Right-view keys of a pass, by how they are read: disparity iff the key
+// carries this call's tag and the pixel is inside the border.
+// census_match_kernel's (atomicMin): tag | cost << 16 | disparity.
+struct MinKeys {
+    uint32_t tag;
+    template <typename T>
+    __device__ __forceinline__ T code(uint32_t key, bool inside) const {
+        const bool ok = inside && (key & (0x1Fu << kRLTagShift)) == tag && ((key >> 16) & 0x7FFu) < 2047u;
+        return disp_code<T>(ok, key & 0xFFFFu);
+    }
+};
+// The tensor-core pass's (atomicMax): tag | order of the key, whose low byte
+// is minus the disparity relative to dmin.
+struct MaxKeys {
+    uint32_t tag;
+    int dmin;
+    template <typename T>
+    __device__ __forceinline__ T code(uint32_t key, bool inside) const {
+        return disp_code<T>(inside && (key & (0x1Fu << kRLTagShift)) == tag, ((0u - key) & 255u) + uint32_t(dmin));
+    }
+};
 // Disparity of a map code (the cross-check's reading: U8 0xFF and U16
 // codes outside CT_DISP_FIRST .. CT_DISP_LAST are not disparities).
 template <typename T>
@@ -679,8 +696,8 @@ __device__ __forceinline__ bool map_disp(T v, int& d) {
 // confirms it as crosscheck_kernel reads the right-view map (U16: the codes
 // within tol; U8: a disparity within tol), from the keys directly. The keys
 // stay in place.
-template <typename T>
-__global__ void __launch_bounds__(128) rl_check_kernel(const uint32_t* keys, size_t kpitch, uint32_t tag, int W,
+template <typename T, typename Keys>
+__global__ void __launch_bounds__(128) rl_check_kernel(const uint32_t* keys, size_t kpitch, Keys how, int W,
                                                        int H, int r, T* rl_out, size_t rl_pitch_b, const T* lr,
                                                        size_t lr_pitch_b, T* ck_out, size_t ck_pitch_b, int tol) {
     constexpr int PX = 16 / sizeof(T);
@@ -708,7 +725,7 @@ __global__ void __launch_bounds__(128) rl_check_kernel(const uint32_t* keys, siz
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int x = x0 + 4 * q + i;
-                o.v[4 * q + i] = rl_code<T>(kk[i], tag, yin && x >= r && x < W - r);
+                o.v[4 * q + i] = how.template code<T>(kk[i], yin && x >= r && x < W - r);
             }
         }
         if (full) *reinterpret_cast<uint4*>(orow + x0) = o.q;
@@ -733,7 +750,7 @@ __global__ void __launch_bounds__(128) rl_check_kernel(const uint32_t* keys, siz
                 const int xo = x - d;
                 out = sizeof(T) == 1 ? T(0xFF) : T(CT_DISP_INCONSISTENT);
                 if (xo >= 0 && xo < W) {
-                    const T vo = rl_code<T>(__ldg(krow + xo), tag, yin && xo >= r && xo < W - r);
+                    const T vo = how.template code<T>(__ldg(krow + xo), yin && xo >= r && xo < W - r);
                     int dd;
                     // U16: raw codes compared (CrossCheckDisparityMaps.cu:94);
                     // U8: only a disparity confirms
