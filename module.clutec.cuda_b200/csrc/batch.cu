@@ -8,24 +8,24 @@
 //   2. one census launch: every CTA is one 64 x 32 census tile of one image of
 //      one pair (census_tile.cuh), found by a scan of per-pair prefix counts;
 //   3. one persistent matching launch, one CTA per SM: each CTA takes work
-//      items (pair, strip, column tile, disparity block) from a global atomic
-//      counter, largest pairs first, and runs the fused census match tile
-//      (census_match.cuh, left-to-right with the right view's winners bid
-//      into the pair's right-view key plane) on the pair's pair-planar
-//      descriptors. The last CTA of a (strip, column tile) group merges the
-//      disparity blocks; the last group of a strip (all column tiles) runs
-//      the cross-check of that strip into the caller's map from the left map
-//      and the right-view keys, then resets the strip's keys. Counters reset
-//      themselves, so nothing waits on anything.
+//      items (pair, strip, tile pair) from a global atomic counter, the
+//      longest first, and runs the tensor-core census tile (census_tc.cuh: the
+//      left map, and the right view's winners bid into the pair's right-view
+//      key plane) on the pair's descriptors;
+//   4. one cross-check launch, a CTA a row of a pair: the caller's map from the
+//      left map and the right-view keys, which it then resets.
 // Results are bit-identical to processing each pair alone: every tile's
 // arithmetic is the same and the winner-take-all keys are order-free.
 #include "ct_internal.h"
 #include "ct_device.cuh"
 #include "census_match.cuh"
+#include "census_tc.cuh"
 #include "census_tile.cuh"
 
 #include <algorithm>
+#include <functional>
 #include <map>
+#include <queue>
 #include <tuple>
 #include <vector>
 
@@ -37,16 +37,16 @@ constexpr int kMaxPairs = 256;
 // Device-side description of one pair (fixed at configure, except the
 // per-call fields at the end, rewritten by every process call).
 struct PairDev {
-    int W, H, D, th, tiles_x, strips, zc, tol;
+    int W, H, D, th, tiles_x, strips, tol;
+    int mo, n, lstep, rstep;                 // tile pair (ctc::Shape)
     int census_tx, census_ty, census_item0;  // census tiles per image, prefix over census CTAs
     int match_item0, match_items;            // prefix over matching items
-    uint64_t* desc[2];                       // pair-planar descriptors: left, right
-    uint32_t* keys;                          // zc left-to-right key planes
-    uint32_t* counters;                      // strips x tiles_x group counters
-    uint32_t* strip_counter;                 // strips
+    int row0;                                // prefix over rows
+    uint64_t* desc[2];                       // row-major descriptors: left, right
+    size_t desc_pitch;                       // elements
     uint16_t* map;                           // U16 left-to-right disparity map
     size_t map_pitch;                        // bytes
-    uint32_t* rl_keys;                       // right-view keys (tag 0), 0xFFFFFFFF between calls
+    uint32_t* rl_keys;                       // right-view keys (kTag), 0 between calls
     size_t rl_pitch;                         // words
     // per call
     void* out;
@@ -54,6 +54,8 @@ struct PairDev {
     int out_type;
     int pad;
 };
+
+constexpr uint32_t kTag = 1u << cm::kRLTagShift;
 
 // Per-call tensor maps of the caller's images, 64-byte aligned in device memory.
 struct alignas(64) CallMaps {
@@ -65,12 +67,13 @@ __device__ __forceinline__ void tmap_acquire(const CUtensorMap* m) {
                  : "memory");
 }
 
-__device__ __forceinline__ int find_pair(const PairDev* pairs, int n, int item, bool census) {
-    int lo = 0, hi = n - 1;  // last pair whose first item <= item
+// Last pair whose first item (PairDev member FIRST) is <= item.
+template <int PairDev::*FIRST>
+__device__ __forceinline__ int find_pair(const PairDev* pairs, int n, int item) {
+    int lo = 0, hi = n - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        const int first = census ? pairs[mid].census_item0 : pairs[mid].match_item0;
-        if (first <= item) lo = mid;
+        if (pairs[mid].*FIRST <= item) lo = mid;
         else hi = mid - 1;
     }
     return lo;
@@ -80,7 +83,7 @@ __global__ void __launch_bounds__(census::kNT) census_batch_kernel(const PairDev
                                                                     const CallMaps* maps, int32_t* status) {
     __shared__ __align__(128) census::TileSmem sm;
     const int item = blockIdx.x;
-    const int p = find_pair(pairs, n, item, true);
+    const int p = find_pair<&PairDev::census_item0>(pairs, n, item);
     const PairDev& P = pairs[p];
     const int local = item - P.census_item0;
     const int per_img = P.census_tx * P.census_ty;
@@ -93,51 +96,68 @@ __global__ void __launch_bounds__(census::kNT) census_batch_kernel(const PairDev
     if (threadIdx.x == 0) tmap_acquire(tm);
     __syncthreads();
     census::census_tile(tm, P.W, P.H, (t % P.census_tx) * census::kTX, (t / P.census_tx) * census::kTY,
-                        P.desc[img], 0, 1, status, sm);
+                        P.desc[img], P.desc_pitch, 0, status, sm);
 }
 
-// Cross-check of rows [y0, y1) of a pair from its U16 left map and the
-// right-view keys into the caller's map (CrossCheckDisparityMaps.cu:63-110
-// rule, left-to-right: the right view's code at x - d, as its map would hold
-// it, within tol of the left code); then the rows' keys are reset.
-__device__ void crosscheck_rows(const PairDev& P, int y0, int y1, int nt) {
-    const int W = P.W;
-    for (int idx = threadIdx.x; idx < (y1 - y0) * W; idx += nt) {
-        const int y = y0 + idx / W, x = idx % W;
-        const uint16_t v = __ldcg(reinterpret_cast<const uint16_t*>(
-                                      reinterpret_cast<const char*>(P.map) + (size_t)y * P.map_pitch) + x);
-        const bool disp = v >= CT_DISP_FIRST && v <= CT_DISP_LAST;
-        bool keep = false;
-        if (disp) {
-            const int d = int(v) - 1, xo = x - d;
-            if (xo >= 0 && xo < W) {
-                const bool inside = y >= cm::kAR && y < P.H - cm::kAR && xo >= cm::kAR && xo < W - cm::kAR;
-                const uint16_t vo = cm::MinKeys{0u}.code<uint16_t>(__ldcg(P.rl_keys + (size_t)y * P.rl_pitch + xo), inside);
+// Cross-check of one row of a pair from its U16 left map and the right-view
+// keys into the caller's map (CrossCheckDisparityMaps.cu:63-110 rule,
+// left-to-right: the right view's code at x - d, as its map would hold it,
+// within tol of the left code), 8 pixels a thread; then the row's keys are
+// reset. A launch of its own: run by the matching CTA that finished a strip,
+// it kept that CTA's tensor core idle for a strip's dependent loads.
+constexpr int kCheckT = 128;
+__global__ void __launch_bounds__(kCheckT) check_batch_kernel(const PairDev* pairs, int n) {
+    const int p = find_pair<&PairDev::row0>(pairs, n, blockIdx.x);
+    const PairDev& P = pairs[p];
+    const int W = P.W, y = blockIdx.x - P.row0;
+    const bool yin = y >= cm::kAR && y < P.H - cm::kAR;
+    const cm::MaxKeys how{kTag, 0};
+    const uint16_t* map = reinterpret_cast<const uint16_t*>(reinterpret_cast<const char*>(P.map) + (size_t)y * P.map_pitch);
+    uint32_t* keys = P.rl_keys + (size_t)y * P.rl_pitch;
+    char* row = static_cast<char*>(P.out) + (size_t)y * P.out_pitch;
+    for (int x0 = 8 * threadIdx.x; x0 < W; x0 += 8 * kCheckT) {
+        // the map's and the caller's rows are 16-byte aligned; the map's pitch
+        // is a multiple of 256
+        const uint4 q = *reinterpret_cast<const uint4*>(map + x0);
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        uint32_t o16[4] = {0, 0, 0, 0}, o8[2] = {0, 0};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint16_t v = uint16_t(w[i >> 1] >> (16 * (i & 1)));
+            const bool disp = v >= CT_DISP_FIRST && v <= CT_DISP_LAST && x0 + i < W;
+            const int xo = x0 + i - (int(v) - 1);
+            bool keep = false;
+            if (disp && xo >= 0 && xo < W) {
+                const uint16_t vo = how.code<uint16_t>(keys[xo], yin && xo >= cm::kAR && xo < W - cm::kAR);
                 keep = abs(int(vo) - int(v)) <= P.tol;  // raw codes, CrossCheckDisparityMaps.cu:94
             }
+            o16[i >> 1] |= uint32_t(keep ? v : (disp ? uint16_t(CT_DISP_INCONSISTENT) : v)) << (16 * (i & 1));
+            o8[i >> 2] |= uint32_t(keep ? uint8_t(v - 1) : uint8_t(0xFF)) << (8 * (i & 3));
         }
-        char* row = static_cast<char*>(P.out) + (size_t)y * P.out_pitch;
         if (P.out_type == CT_PIX_U8) {
-            reinterpret_cast<uint8_t*>(row)[x] = keep ? uint8_t(v - 1) : uint8_t(0xFF);
+            uint8_t* o = reinterpret_cast<uint8_t*>(row) + x0;
+            if (x0 + 8 <= W) *reinterpret_cast<uint2*>(o) = make_uint2(o8[0], o8[1]);
+            else
+                for (int i = 0; x0 + i < W; ++i) o[i] = uint8_t(o8[i >> 2] >> (8 * (i & 3)));
         } else {
-            reinterpret_cast<uint16_t*>(row)[x] = keep ? v : (disp ? uint16_t(CT_DISP_INCONSISTENT) : v);
+            uint16_t* o = reinterpret_cast<uint16_t*>(row) + x0;
+            if (x0 + 8 <= W) *reinterpret_cast<uint4*>(o) = make_uint4(o16[0], o16[1], o16[2], o16[3]);
+            else
+                for (int i = 0; x0 + i < W; ++i) o[i] = uint16_t(o16[i >> 1] >> (16 * (i & 1)));
         }
     }
-    __syncthreads();  // every read of the rows' keys done
-    for (int idx = threadIdx.x; idx < (y1 - y0) * W; idx += nt)
-        P.rl_keys[(size_t)(y0 + idx / W) * P.rl_pitch + idx % W] = 0xFFFFFFFFu;
+    __syncthreads();  // every read of the row's keys done
+    for (int i = 4 * threadIdx.x; i < int(P.rl_pitch); i += 4 * kCheckT)
+        *reinterpret_cast<uint4*>(keys + i) = make_uint4(0, 0, 0, 0);
 }
 
-__global__ void __launch_bounds__(cm::Var<4>::kNT, 1)
-    match_batch_kernel(const PairDev* pairs, int n, int total_items, const CUtensorMap* match_maps,
-                       unsigned* queue, int32_t* status) {
-    using namespace cm;
-    constexpr int NT = Var<4>::kNT;
+__global__ void __launch_bounds__(ctc::kNT, 1)
+    match_batch_kernel(const PairDev* pairs, int n, int total_items, unsigned* queue, int32_t* status) {
+    constexpr int NT = ctc::kNT;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const Smem sm(smem_raw);
-    __shared__ int s_item, s_last;
-    init_barriers(sm);
-    uint32_t par[2] = {0, 0};
+    __shared__ int s_item;
+    ctc::Cta c(smem_raw);
+    ctc::cta_begin(c);
     const int tid = threadIdx.x;
     for (;;) {
         if (tid == 0) s_item = int(atomicAdd(queue, 1u));
@@ -145,52 +165,28 @@ __global__ void __launch_bounds__(cm::Var<4>::kNT, 1)
         const int item = s_item;
         __syncthreads();
         if (item >= total_items) break;
-        const int p = find_pair(pairs, n, item, false);
+        const int p = find_pair<&PairDev::match_item0>(pairs, n, item);
         const PairDev& P = pairs[p];
-        int local = item - P.match_item0;
-        if (local < 0 || local >= P.match_items || P.match_items != P.strips * P.tiles_x * P.zc) {
+        const int local = item - P.match_item0;
+        if (local < 0 || local >= P.match_items || P.match_items != P.strips * P.tiles_x) {
             if (tid == 0) dev::report(status, CT_EINTERNAL);  // table inconsistent
             break;
         }
-        // disparity blocks of one group are consecutive items, so the group's
-        // CTAs run close together and the merging one finds its inputs in L2
-        const Tile t{(local / P.zc) % P.tiles_x, local / (P.zc * P.tiles_x), local % P.zc, P.tiles_x, P.zc};
-        MatchArgs a{};
-        a.W = P.W; a.H = P.H; a.D = P.D; a.th = P.th;
-        a.keys = P.keys;
-        a.counters = P.counters;
-        a.merge_last = 1;
+        const int by = local / P.tiles_x;
+        ctc::Args a{};
+        a.W = P.W; a.H = P.H; a.D = P.D;
+        a.mo = P.mo; a.n = P.n; a.th = P.th;
+        a.lstep = P.lstep; a.rstep = P.rstep;
+        a.left = P.desc[0]; a.right = P.desc[1];
+        a.pitch = P.desc_pitch;
         a.out = P.map; a.out_pitch = P.map_pitch; a.out_type = CT_PIX_U16;
+        a.r_keys = P.rl_keys;
+        a.key_pitch = P.rl_pitch;
+        a.tag = kTag;
         a.status = status;
-        a.rl_keys = P.rl_keys;  // tag 0: the strip's cross-check resets the keys it read
-        a.rl_pitch = P.rl_pitch;
-        a.rl_tag = 0u;
-        const CUtensorMap* tb = &match_maps[p * 2 + 0];
-        const CUtensorMap* tm = &match_maps[p * 2 + 1];
-        if (tid == 0) {  // maps written by a host copy: make them visible to the TMA unit
-            tmap_acquire(tb);
-            tmap_acquire(tm);
-        }
-        const TileResult res = run_tile<0, 4, false, true>(tb, tm, a, t, sm, par);
-        if (res.aborted) break;  // status already set; the CTA stops taking work
-        if (res.group_done) {
-            // one more finished column tile group of this strip
-            if (tid == 0) {
-                __threadfence();
-                unsigned* sc = reinterpret_cast<unsigned*>(&P.strip_counter[t.by]);
-                const unsigned prev = atomicAdd(sc, 1u);
-                s_last = prev == unsigned(P.tiles_x) - 1;
-                if (s_last) *sc = 0u;
-            }
-            __syncthreads();
-            if (s_last) {
-                __threadfence();
-                const int y0 = t.by * P.th;
-                crosscheck_rows(P, y0, min(P.H, y0 + P.th), NT);
-            }
-            __syncthreads();
-        }
+        if (!ctc::run_tile(c, a, local % P.tiles_x, by)) break;  // status already set; the CTA takes no more work
     }
+    ctc::cta_end(c);
 }
 
 // ---------------------------------------------------------------------------
@@ -250,11 +246,10 @@ struct BatchHandle : ct_handle {
     std::vector<ct_batch_shape> shapes;
     std::vector<PairDev> pairs;          // host copy (per-call fields filled per call)
     std::vector<int> order;              // pair index -> position in the device table
-    int total_census = 0, total_match = 0;
+    int total_census = 0, total_match = 0, total_rows = 0;
     unsigned char* arena = nullptr;      // one device allocation for all scratch
     PairDev* d_pairs = nullptr;
     CallMaps* d_maps = nullptr;
-    CUtensorMap* d_match_maps = nullptr;
     unsigned* d_queue = nullptr;
     Staging stage[kSlots];               // process calls
     int next_slot = 0;
@@ -305,21 +300,71 @@ int enqueue(BatchHandle* h, Staging& st, bool record, cudaStream_t s) {
     CT_CUDA_TRY(cudaMemsetAsync(h->d_queue, 0, sizeof(unsigned), s));
     census_batch_kernel<<<h->total_census, census::kNT, 0, s>>>(h->d_pairs, h->n, h->d_maps, h->d_status);
     CT_LAUNCH_CHECK();
-    match_batch_kernel<<<h->sms, cm::Var<4>::kNT, cm::smem_bytes_rl(), s>>>(h->d_pairs, h->n, h->total_match,
-                                                                        h->d_match_maps, h->d_queue, h->d_status);
+    match_batch_kernel<<<std::min(h->sms, h->total_match), ctc::kNT, ctc::kSmemBytes, s>>>(
+        h->d_pairs, h->n, h->total_match, h->d_queue, h->d_status);
+    CT_LAUNCH_CHECK();
+    check_batch_kernel<<<h->total_rows, kCheckT, 0, s>>>(h->d_pairs, h->n);
     CT_LAUNCH_CHECK();
     return CT_OK;
 }
 
-// Lays out the table (largest pairs first), item prefixes and scratch for the
-// current shapes and strip heights; (re)creates the fixed tensor maps.
+// Strip heights keep the form 5 k + 1 that callers of ct_batch_strip_height know.
+constexpr int strip_form(int th) { return th + (6 - th % 5) % 5; }
+
+// Strip heights: the same target for every pair, the one whose items finish
+// first when handed out longest first. An item takes its rows, the first
+// window and the start of its pipeline (about 7 rows' worth) times the tile
+// pair's cost of a row. With very many items their order no longer matters and
+// tall strips repeat fewer rows.
+std::vector<int> pick_strips(const std::vector<ct_batch_shape>& shapes, int sms) {
+    const int n = int(shapes.size());
+    std::vector<ctc::Shape> sh(n);
+    for (int i = 0; i < n; ++i) sh[i] = ctc::pick_shape(shapes[i].width, shapes[i].disp_count);
+    std::vector<int> best(n), th(n);
+    double best_time = -1;
+    for (int target : {8, 12, 16, 24, 32, 48, 64, 80, 96, 128, 160, 192, 256}) {
+        std::vector<std::pair<double, long>> items;  // cost, how many
+        long count = 0;
+        double total = 0;
+        for (int i = 0; i < n; ++i) {
+            const int strips = (shapes[i].height + target - 1) / target;
+            th[i] = strip_form((shapes[i].height + strips - 1) / strips);
+            const double cost = (std::min(th[i], shapes[i].height) + 7) * sh[i].row_cost;
+            const long k = long((shapes[i].height + th[i] - 1) / th[i]) * sh[i].tiles_x;
+            items.push_back({cost, k});
+            count += k;
+            total += cost * k;
+        }
+        double time = total / sms;
+        if (count <= 64L * sms) {
+            std::sort(items.begin(), items.end(), std::greater<>());
+            std::priority_queue<double, std::vector<double>, std::greater<>> cta;
+            for (int k = 0; k < sms; ++k) cta.push(0.0);
+            for (auto& it : items)
+                for (long k = 0; k < it.second; ++k) {
+                    const double t = cta.top() + it.first;
+                    cta.pop();
+                    cta.push(t);
+                    time = std::max(time, t);
+                }
+        }
+        if (best_time < 0 || time < best_time) {
+            best_time = time;
+            best = th;
+        }
+    }
+    return best;
+}
+
+// Lays out the table (longest items first), item prefixes and scratch for the
+// current shapes and strip heights.
 int layout(BatchHandle* h, const std::vector<int>& th) {
     const int n = h->n;
     std::vector<int> idx(n);
     for (int i = 0; i < n; ++i) idx[i] = i;
     auto cost = [&](int i) {
-        const ct_batch_shape& s = h->shapes[i];
-        return double(s.width) * s.height * ((s.disp_count + cm::kDPC - 1) / cm::kDPC);
+        return (std::min(th[i], h->shapes[i].height) + 7) *
+               ctc::pick_shape(h->shapes[i].width, h->shapes[i].disp_count).row_cost;
     };
     std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return cost(a) > cost(b); });
     h->order.assign(n, 0);
@@ -327,65 +372,56 @@ int layout(BatchHandle* h, const std::vector<int>& th) {
     // sizes
     size_t bytes = 0;
     auto take = [&](size_t b) { const size_t o = bytes; bytes += (b + 255) / 256 * 256; return o; };
-    struct Off { size_t desc[2], keys, cnt, strip, map, rl; };
+    struct Off { size_t desc[2], map, rl; };
     std::vector<Off> off(n);
     h->pairs.assign(n, PairDev{});
-    int census0 = 0, match0 = 0;
+    int census0 = 0, match0 = 0, row0 = 0;
     for (int k = 0; k < n; ++k) {
         const int i = idx[k];
         const ct_batch_shape& s = h->shapes[i];
         PairDev& P = h->pairs[k];
         P.W = s.width; P.H = s.height; P.D = s.disp_count; P.th = th[i];
-        P.tiles_x = (P.W + cm::kTWO - 1) / cm::kTWO;
+        const ctc::Shape shape = ctc::pick_shape(P.W, P.D);
+        P.mo = shape.mo; P.n = shape.n; P.lstep = shape.lstep; P.rstep = shape.rstep;
+        P.tiles_x = shape.tiles_x;
         P.strips = (P.H + P.th - 1) / P.th;
-        P.zc = (P.D + cm::kDPC - 1) / cm::kDPC;
         P.tol = h->tol;
         P.census_tx = (P.W + census::kTX - 1) / census::kTX;
         P.census_ty = (P.H + census::kTY - 1) / census::kTY;
         P.census_item0 = census0;
         census0 += 2 * P.census_tx * P.census_ty;
         P.match_item0 = match0;
-        P.match_items = P.strips * P.tiles_x * P.zc;
+        P.match_items = P.strips * P.tiles_x;
         match0 += P.match_items;
+        P.row0 = row0;
+        row0 += P.H;
         P.map_pitch = ((size_t)P.W * 2 + 255) / 256 * 256;
         Off& o = off[k];
-        for (int v = 0; v < 2; ++v) o.desc[v] = take(cm::planar_pitch(P.W) * P.H * 8);
-        o.keys = take((size_t)P.zc * P.W * P.H * 4);
-        o.cnt = take((size_t)P.strips * P.tiles_x * 4);
+        P.desc_pitch = ((size_t)P.W + 1) / 2 * 2;  // 16-byte rows
+        for (int v = 0; v < 2; ++v) o.desc[v] = take(P.desc_pitch * P.H * 8);
         o.map = take(P.map_pitch * P.H);
         P.rl_pitch = cm::rl_pitch_words(P.W);
         o.rl = take(P.rl_pitch * P.H * 4);
-        o.strip = take((size_t)P.strips * 4);
     }
     const size_t o_pairs = take(sizeof(PairDev) * n), o_maps = take(sizeof(CallMaps) * n);
-    const size_t o_mmaps = take(sizeof(CUtensorMap) * 2 * n), o_queue = take(256);
+    const size_t o_queue = take(256);
     cudaFree(h->arena);
     h->arena = nullptr;
     if (cudaMalloc(&h->arena, bytes) != cudaSuccess) return fail(CT_ENOMEM, "batch scratch (%zu bytes)", bytes);
-    CT_CUDA_TRY(cudaMemset(h->arena, 0, bytes));  // counters start at 0
+    CT_CUDA_TRY(cudaMemset(h->arena, 0, bytes));  // right-view keys start at 0
     unsigned char* A = h->arena;
     for (int k = 0; k < n; ++k) {
         PairDev& P = h->pairs[k];
         for (int v = 0; v < 2; ++v) P.desc[v] = reinterpret_cast<uint64_t*>(A + off[k].desc[v]);
-        P.keys = reinterpret_cast<uint32_t*>(A + off[k].keys);
-        P.counters = reinterpret_cast<uint32_t*>(A + off[k].cnt);
         P.map = reinterpret_cast<uint16_t*>(A + off[k].map);
         P.rl_keys = reinterpret_cast<uint32_t*>(A + off[k].rl);
-        CT_CUDA_TRY(cudaMemset(P.rl_keys, 0xFF, P.rl_pitch * P.H * 4));
-        P.strip_counter = reinterpret_cast<uint32_t*>(A + off[k].strip);
     }
     h->d_pairs = reinterpret_cast<PairDev*>(A + o_pairs);
     h->d_maps = reinterpret_cast<CallMaps*>(A + o_maps);
-    h->d_match_maps = reinterpret_cast<CUtensorMap*>(A + o_mmaps);
     h->d_queue = reinterpret_cast<unsigned*>(A + o_queue);
     h->total_census = census0;
     h->total_match = match0;
-    std::vector<CUtensorMap> mm(2 * n);  // left as base, right as match
-    for (int k = 0; k < n; ++k) {
-        const PairDev& P = h->pairs[k];
-        if (int rc = cm::make_planar_maps(&mm[2 * k + 0], &mm[2 * k + 1], P.desc[0], P.desc[1], P.W, P.H)) return rc;
-    }
-    CT_CUDA_TRY(cudaMemcpy(h->d_match_maps, mm.data(), sizeof(CUtensorMap) * 2 * n, cudaMemcpyHostToDevice));
+    h->total_rows = row0;
     if (h->graph_exec) {
         cudaGraphExecDestroy(h->graph_exec);
         h->graph_exec = nullptr;
@@ -425,16 +461,13 @@ int ct_batch_configure(ct_handle* hh, int32_t device, const ct_batch_shape* shap
     if (int rc = use_device(device)) return rc;
     h->device = device;
     if (int rc = h->init_status()) return rc;
-    CT_CUDA_TRY(cm::prepare_census_match());
     CT_CUDA_TRY(cudaFuncSetAttribute(match_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(cm::smem_bytes_rl())));
+                                     ctc::kSmemBytes));
     h->sms = sm_count(device);
     h->n = n;
     h->tol = tol;
     h->shapes.assign(shapes, shapes + n);
-    std::vector<int> th(n);
-    for (int i = 0; i < n; ++i)
-        th[i] = cm::pick_strip_height(shapes[i].width, shapes[i].height, shapes[i].disp_count, h->sms);
+    const std::vector<int> th = pick_strips(h->shapes, h->sms);
     if (int rc = layout(h, th)) return rc;
     for (Staging& st : h->stage)
         if (int rc = st.alloc(n)) return rc;
@@ -499,8 +532,8 @@ int ct_batch_autotune(ct_handle* hh, const ct_batch_item* items, int32_t n, ct_s
     for (auto& g : groups) {
         const int base = th[g.second[0]];
         int best_th = base;
-        for (int cand : {base / 2 - (base / 2 + 4) % 10, base - 40, base + 40, 26, 66}) {
-            if (cand < 16 || cand > 506 || cand == best_th || (cand + 4) % 5 != 0) continue;
+        for (int cand : {strip_form(base / 2), strip_form(base * 2), strip_form(base * 3 / 2), 31, 66}) {
+            if (cand < 6 || cand > h->shapes[g.second[0]].height || cand == best_th) continue;
             for (int i : g.second) th[i] = cand;
             if ((rc = layout(h, th))) goto done;
             float t = 0.f;

@@ -99,6 +99,19 @@ __global__ void to_planar_kernel(const uint64_t* src, size_t src_pitch, uint64_t
     if (x < W && y < H) dst[cm::planar_index(x, y, W)] = src[(size_t)y * src_pitch + x];
 }
 
+// One tile pair a CTA: grid (pairs, strips).
+__global__ void __launch_bounds__(ctc::kNT, 1) census_tc_kernel(const ctc::Args a) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    ctc::Cta c(smem_raw);
+    ctc::cta_begin(c);
+    // launched with programmatic stream serialisation: the descriptors are
+    // complete after this
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    ctc::run_tile(c, a, blockIdx.x, blockIdx.y);
+    ctc::cta_end(c);
+}
+
 // ---------------------------------------------------------------------------
 // CensusTransform::CDriver
 // ---------------------------------------------------------------------------
@@ -294,7 +307,7 @@ int census_process_tc(BmCensusHandle* h, const ct_image* lr, const ct_image* dis
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, ctc::census_tc_kernel, a));
+    CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, census_tc_kernel, a));
     CT_LAUNCH_CHECK();
     if (!need_r) return CT_OK;
     return rl_check(h, (disp_rl ? disp_rl : disp_checked)->type, cm::MaxKeys{tag, a.dmin}, lr, disp_rl, disp_checked, tol, s);
@@ -454,7 +467,7 @@ int ct_bm_census_configure(ct_handle* hh, int32_t device, const ct_format* fmt, 
     h->use_tc_right = tc_faster(W, H, p->disp_count, false);
     h->tc = ctc::pick_shape(W, p->disp_count);
     h->tc_rows = ctc::pick_rows(H, h->tc.tiles_x, sm_count(device));
-    CT_CUDA_TRY(cudaFuncSetAttribute(ctc::census_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CT_CUDA_TRY(cudaFuncSetAttribute(census_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      ctc::kSmemBytes));
     h->fmt = *fmt;  // left_desc() / right_desc() below depend on the height
     h->th = cm::pick_strip_height(W, H, p->disp_count, sm_count(device));

@@ -52,6 +52,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "census_match.cuh"
 #include "ct_device.cuh"
@@ -103,6 +104,7 @@ struct Args {
 
 struct Shape {
     int mo, n, lstep, rstep, tiles_x;  // tiles_x: pairs of tiles in a strip
+    double row_cost;                   // cycles of a pair's row (estimate)
 };
 
 // Shape of the tile pair: neighbouring column tiles, or (from about 150
@@ -127,7 +129,8 @@ inline Shape pick_shape(int W, int D) {
         s.rstep = split ? s.n : s.mo;
         const double mma = 20.0 * std::max(s.n / 2, 32 + s.n / 4);
         const double alu = 2.0 * (4 * ((std::min(s.n, D + 31) + kPiece - 1) / kPiece) * 55.0 + 300.0);
-        const double cost = s.tiles_x * std::max(mma, alu);
+        s.row_cost = std::max(mma, alu);
+        const double cost = s.tiles_x * s.row_cost;
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
             best = s;
@@ -588,48 +591,62 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
                 fence_before();
                 read_arrive(t);
             }
-            for (; p < pieces; p += 4) {
+            auto reduce_pieces = [&](auto pair) {
+                constexpr bool kTwo = decltype(pair)::value;
                 const int na = min(c_lo + kPiece * p, a.n - kPiece);
-                const int nb = p + 2 < pieces ? min(c_lo + kPiece * (p + 2), a.n - kPiece) : na;
+                const int nb = min(c_lo + kPiece * (p + 2), a.n - kPiece);
                 float v[4][10], wa[10], wb[10];
                 ld_piece(tq + uint32_t(na), v);
-                reduce(v, wa);
-                ld_piece(tq + uint32_t(nb), v);
+                if constexpr (kTwo) {
+                    reduce(v, wa);
+                    ld_piece(tq + uint32_t(nb), v);
+                }
                 if (p + 4 >= pieces) {
                     fence_before();
                     read_arrive(t);
                 }
-                reduce(v, wb);
-                if (a.r_keys) {
-                    // The column maxima over the 8 lanes of equal t % 4,
-                    // halving the columns a lane keeps while it can: of
-                    // w[0..3], w[8] and w[4..7], w[9], then of the four, then
-                    // of the two.
-                    float ua[4], ub[4];
+                if constexpr (kTwo) reduce(v, wb);
+                else reduce(v, wa);
+                if (!a.r_keys) return;
+                // The column maxima over the 8 lanes of equal t % 4, halving
+                // the columns a lane keeps while it can: of w[0..3], w[8] and
+                // w[4..7], w[9], then of the four, then of the two. Both
+                // pieces level by level, so that one's shuffles cover the
+                // other's latency.
+                float ua[4], ub[4], za, zb;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) ua[j] = halve(wa[j], wa[j + 4], f4, 16);
-                    float za = halve(wa[8], wa[9], f4, 16);
+                for (int j = 0; j < 4; ++j) ua[j] = halve(wa[j], wa[j + 4], f4, 16);
+                za = halve(wa[8], wa[9], f4, 16);
+                if constexpr (kTwo) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) ub[j] = halve(wb[j], wb[j + 4], f4, 16);
-                    float zb = halve(wb[8], wb[9], f4, 16);
-                    ua[0] = halve(ua[0], ua[1], f3, 8);
-                    ua[2] = halve(ua[2], ua[3], f3, 8);
-                    za = fmaxf(za, __shfl_xor_sync(0xffffffffu, za, 8));
+                    zb = halve(wb[8], wb[9], f4, 16);
+                }
+                ua[0] = halve(ua[0], ua[1], f3, 8);
+                ua[2] = halve(ua[2], ua[3], f3, 8);
+                za = fmaxf(za, __shfl_xor_sync(0xffffffffu, za, 8));
+                if constexpr (kTwo) {
                     ub[0] = halve(ub[0], ub[1], f3, 8);
                     ub[2] = halve(ub[2], ub[3], f3, 8);
                     zb = fmaxf(zb, __shfl_xor_sync(0xffffffffu, zb, 8));
-                    ua[0] = halve(ua[0], ua[2], f2, 4);
-                    za = fmaxf(za, __shfl_xor_sync(0xffffffffu, za, 4));
+                }
+                ua[0] = halve(ua[0], ua[2], f2, 4);
+                za = fmaxf(za, __shfl_xor_sync(0xffffffffu, za, 4));
+                if constexpr (kTwo) {
                     ub[0] = halve(ub[0], ub[2], f2, 4);
                     zb = fmaxf(zb, __shfl_xor_sync(0xffffffffu, zb, 4));
-                    float* d = put_kr + (s & (kRowsR - 1)) * (4 * kKeyN);
-                    d[na + col0] = ua[0];
-                    d[nb + col0] = ub[0];
-                    if (!(lane & 12)) {
-                        d[na + col1] = za;
-                        d[nb + col1] = zb;
-                    }
                 }
+                float* d = put_kr + (s & (kRowsR - 1)) * (4 * kKeyN);
+                d[na + col0] = ua[0];
+                if constexpr (kTwo) d[nb + col0] = ub[0];
+                if (!(lane & 12)) {
+                    d[na + col1] = za;
+                    if constexpr (kTwo) d[nb + col1] = zb;
+                }
+            };
+            for (; p < pieces; p += 4) {
+                if (p + 2 < pieces) reduce_pieces(std::true_type{});
+                else reduce_pieces(std::false_type{});
             }
             // row s - 2: every warp wrote its keys before it read row s - 1's
             // accumulator, which the MMAs of this row waited for
@@ -663,19 +680,6 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
     const bool failed = __syncthreads_or(polls == 0);
     if (failed && tid == 0) dev::report(a.status, CT_ETIMEOUT);
     return !failed;
-}
-
-// One tile pair a CTA: grid (pairs, strips).
-__global__ void __launch_bounds__(kNT, 1) census_tc_kernel(const Args a) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    Cta c(smem_raw);
-    cta_begin(c);
-    // launched with programmatic stream serialisation: the descriptors are
-    // complete after this
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    run_tile(c, a, blockIdx.x, blockIdx.y);
-    cta_end(c);
 }
 
 }  // namespace ctc
