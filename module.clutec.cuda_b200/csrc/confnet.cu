@@ -134,7 +134,6 @@ struct Act {  // per-sample activations and gradient signals, [n][...]
     uint16_t *a1p, *a1pt;  // [n][256]: slot 0 = 0, slots 1..7 = conv1 positions 0..6; [256][ldt]
     uint16_t *a2b, *a2t, *a3b, *a3t;
     uint16_t *dz4b, *dz4t, *dz3b, *dz3t, *dz2b, *dz2t;
-    float* d;              // GEMM output scratch [n][224]
     int ldt;
 };
 constexpr int kQ = 7;   // pooled conv1 positions
@@ -145,6 +144,8 @@ constexpr int kSY = 16;  // samples per CTA
 // conv1 (k=5, stride 5) over the 35 central codes, ReLU, bf16; also the
 // bf16 operand copies of the conv2 GEMMs (forward and weight gradient)
 __global__ void __launch_bounds__(32 * kSY) fwd1_kernel(const uint8_t* x, const float* wq, Act A, int n) {
+    dev::pdl_launch();
+    dev::pdl_wait();
     __shared__ float xs[kSY][kLen];
     const int o = threadIdx.x, sl = threadIdx.y, s = blockIdx.x * kSY + sl;
     for (int k = threadIdx.x; k < kLen; k += 32) xs[sl][k] = s < n ? float(x[(size_t)s * kLen + k]) : 0.f;
@@ -174,136 +175,138 @@ __global__ void __launch_bounds__(32 * kSY) fwd1_kernel(const uint8_t* x, const 
     }
 }
 
-// Epilogue of a forward GEMM (block (32, 8), 8 samples): v = ReLU(d + bias)
-// (bias[col % bmod]; rounded to bf16 when rnd) into f [n][N] and the bf16
-// operand copies b [n][N] and t [N][ldt] when given.
-__global__ void ep_fwd_kernel(const float* d, int N, const float* bias, int bmod, int rnd, float* f, uint16_t* b,
-                              uint16_t* t, int ldt, int n) {
-    const int s = blockIdx.x * 8 + threadIdx.y;
+// A warp a sample, lane l the hidden units l and l + 32: logit, loss,
+// dloss/dlogit (labels may be null: scores only) and, with labels, dz4 = dl *
+// w5 * (a4 > 0) with its bf16 operand copies.
+constexpr int kHeadT = 256;
+__global__ void __launch_bounds__(kHeadT) head_kernel(const float* wq, Act A, const uint8_t* labels, float inv_n,
+                                                      float* scores, int n) {
+    dev::pdl_launch();
+    dev::pdl_wait();
+    const int s = blockIdx.x * (kHeadT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (s >= ((n + 7) & ~7)) return;
-    for (int c = threadIdx.x; c < N; c += 32) {
-        if (s >= n) {
-            if (t) t[(size_t)c * ldt + s] = 0;
-            continue;
-        }
-        float v = fmaxf(d[(size_t)s * N + c] + bias[c % bmod], 0.f);
-        if (rnd) v = bf16r(v);
-        f[(size_t)s * N + c] = v;
-        if (b) b[(size_t)s * N + c] = bf16_bits(v);
-        if (t) t[(size_t)c * ldt + s] = bf16_bits(v);
-    }
-}
-
-// Epilogue of a data-gradient GEMM (block (32, 8)): g = act > 0 ? d : 0 into
-// f [n][N] and the bf16 copies b, t when given.
-__global__ void ep_bwd_kernel(const float* d, int N, const float* act, float* f, uint16_t* b, uint16_t* t, int ldt,
-                              int n) {
-    const int s = blockIdx.x * 8 + threadIdx.y;
-    if (s >= ((n + 7) & ~7)) return;
-    for (int c = threadIdx.x; c < N; c += 32) {
-        if (s >= n) {
-            if (t) t[(size_t)c * ldt + s] = 0;
-            continue;
-        }
-        const size_t k = (size_t)s * N + c;
-        const float g = act[k] > 0.f ? d[k] : 0.f;
-        f[k] = g;
-        if (b) b[k] = bf16_bits(g);
-        if (t) t[(size_t)c * ldt + s] = bf16_bits(g);
-    }
-}
-
-// one thread per sample: logit, loss, dloss/dlogit (labels may be null: scores only)
-__global__ void head_kernel(const float* wq, Act A, const uint8_t* labels, float inv_n, float* scores, int n) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    float z = wq[kOffB5];
-    for (int h = 0; h < 64; ++h) z = fmaf(wq[kOffW5 + h], A.a4[(size_t)s * 64 + h], z);
-    A.logit[s] = z;
-    const float p = 1.f / (1.f + expf(-z));
-    if (scores) scores[s] = p;
-    if (labels) {
-        const float y = labels[s] ? 1.f : 0.f;
-        A.dl[s] = (p - y) * inv_n;
-        A.loss[s] = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))) - y * z;
-    }
-}
-
-// block (64, 8): dz4 = dl * w5 * (a4 > 0), with its bf16 operand copies
-__global__ void bwd4_kernel(const float* wq, Act A, int n) {
-    const int h = threadIdx.x, s = blockIdx.x * 8 + threadIdx.y;
-    if (s >= ((n + 7) & ~7)) return;
-    if (s >= n) {
-        A.dz4t[(size_t)h * A.ldt + s] = 0;
+    if (s >= n) {  // transposed columns past n read as 0
+        if (labels)
+            for (int h = lane; h < 64; h += 32) A.dz4t[(size_t)h * A.ldt + s] = 0;
         return;
     }
-    const float a = A.a4[(size_t)s * 64 + h];
-    const float g = a > 0.f ? A.dl[s] * wq[kOffW5 + h] : 0.f;
-    A.dz4[(size_t)s * 64 + h] = g;
-    A.dz4b[(size_t)s * 64 + h] = bf16_bits(g);
-    A.dz4t[(size_t)h * A.ldt + s] = bf16_bits(g);
+    const float a0 = A.a4[(size_t)s * 64 + lane], a1 = A.a4[(size_t)s * 64 + 32 + lane];
+    const float w0 = wq[kOffW5 + lane], w1 = wq[kOffW5 + 32 + lane];
+    float z = fmaf(w1, a1, w0 * a0);
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) z += __shfl_xor_sync(0xffffffffu, z, k);
+    z += wq[kOffB5];
+    const float p = 1.f / (1.f + expf(-z));
+    if (lane == 0) {
+        A.logit[s] = z;
+        if (scores) scores[s] = p;
+    }
+    if (!labels) return;
+    const float y = labels[s] ? 1.f : 0.f;
+    const float dl = (p - y) * inv_n;
+    if (lane == 0) {
+        A.dl[s] = dl;
+        A.loss[s] = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))) - y * z;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int h = lane + 32 * k;
+        const float g = (k ? a1 : a0) > 0.f ? dl * (k ? w1 : w0) : 0.f;
+        A.dz4[(size_t)s * 64 + h] = g;
+        A.dz4b[(size_t)s * 64 + h] = bf16_bits(g);
+        A.dz4t[(size_t)h * A.ldt + s] = bf16_bits(g);
+    }
 }
 
 // Weight gradients of one chunk of samples (blockIdx.x) on the CUDA cores,
 // written to part[chunk][param]: conv1 (blockIdx.y 0), the biases of conv2,
 // conv3 and fc1 (1, 2, 3; their weights come from the tensor-core GEMMs)
-// and fc2 (4). 256 threads.
+// and fc2 (4). A lane is a channel, so that a warp reads whole rows, and the
+// 32 warps share the chunk's samples; their sums meet in shared memory in a
+// fixed order. (One thread a parameter walking its chunk's samples was a chain
+// of 1792 dependent loads: 500 us of a 606 us gradient of 8192 samples.)
 constexpr int kChunk = 256;
+constexpr int kWW = 32;  // warps
 
-__global__ void __launch_bounds__(256) wgrad_kernel(const uint8_t* x, Act A, int n, float* part) {
-    const int t = threadIdx.x;
-    const int s0 = blockIdx.x * kChunk, s1 = min(n, s0 + kChunk);
+__global__ void __launch_bounds__(32 * kWW) wgrad_kernel(const uint8_t* x, Act A, int n, float* part) {
+    dev::pdl_launch();
+    dev::pdl_wait();
+    __shared__ float red[kWW][6 * 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int s0 = blockIdx.x * kChunk, cnt = min(n - s0, kChunk);
     float* P = part + (size_t)blockIdx.x * kParams;
+    float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    int used = 0;  // accumulators a lane has
     switch (blockIdx.y) {
-        case 0: {  // w1 (o, j) for t < 160, b1 for 160 <= t < 192
-            if (t >= 192) return;
-            const bool bias = t >= 160;
-            const int o = bias ? t - 160 : t / 5, j = t % 5;
-            float acc = 0.f;
-            for (int s = s0; s < s1; ++s) {
-                for (int q = 0; q < kQ; ++q) {
-                    const float g = A.dm1[(size_t)s * 224 + q * 32 + o];
-                    if (g == 0.f) continue;
-                    if (bias) { acc += g; continue; }
-                    acc = fmaf(g, float(x[(size_t)s * kLen + kCropLo + 5 * q + j]), acc);
-                }
+        case 0: {  // w1[lane][0..4], b1[lane] over the chunk's (sample, position) pairs
+            used = 6;
+            const float* g0 = A.dm1 + (size_t)s0 * 224 + lane;
+            const uint8_t* x0 = x + (size_t)s0 * kLen + kCropLo;
+#pragma unroll 4
+            for (int p = warp; p < cnt * kQ; p += kWW) {
+                const int s = p / kQ, q = p - s * kQ;
+                const float g = g0[p * 32];
+                const uint8_t* xs = x0 + s * kLen + 5 * q;
+#pragma unroll
+                for (int j = 0; j < 5; ++j) acc[j] = fmaf(g, float(xs[j]), acc[j]);
+                acc[5] += g;
             }
-            P[bias ? kOffB1 + o : kOffW1 + t] = acc;
             break;
         }
-        case 1: {  // b2 (w2 by the tensor-core GEMM, tg::kW2T)
-            if (t >= 32) return;
-            float bacc = 0.f;
-            for (int s = s0; s < s1; ++s)
-                for (int r = 0; r < kR; ++r) bacc += A.dz2[(size_t)s * 64 + r * 32 + t];
-            P[kOffB2 + t] = bacc;
+        case 1:  // b2 (w2 by the tensor-core GEMM, tg::kW2T): both positions
+            used = 1;
+#pragma unroll 4
+            for (int p = warp; p < cnt * kR; p += kWW) acc[0] += A.dz2[(size_t)s0 * 64 + p * 32 + lane];
             break;
-        }
-        case 2: {  // b3, and 0 for the taps of w3 that meet no data (taps 2, 3 by tg::kW3T)
-            for (int k = t; k < 32 * 32 * 3; k += 256) {
+        case 2:  // b3, and 0 for the taps of w3 that meet no data (taps 2, 3 by tg::kW3T)
+            used = 1;
+            for (int k = threadIdx.x; k < 32 * 32 * 3; k += 32 * kWW) {
                 const int oi = k / 3, j = k % 3;
                 P[kOffW3 + oi * 5 + (j == 2 ? 4 : j)] = 0.f;
             }
-            if (t >= 32) return;
-            float bacc = 0.f;
-            for (int s = s0; s < s1; ++s) bacc += A.dz3[(size_t)s * 32 + t];
-            P[kOffB3 + t] = bacc;
+#pragma unroll 4
+            for (int p = warp; p < cnt; p += kWW) acc[0] += A.dz3[(size_t)(s0 + p) * 32 + lane];
             break;
-        }
-        case 3: {  // b4 (w4 by tg::kW4)
-            if (t >= 64) return;
-            float bacc = 0.f;
-            for (int s = s0; s < s1; ++s) bacc += A.dz4[(size_t)s * 64 + t];
-            P[kOffB4 + t] = bacc;
+        case 3:  // b4 (w4 by tg::kW4)
+            used = 2;
+#pragma unroll 4
+            for (int p = warp; p < cnt; p += kWW) {
+                const float* d = A.dz4 + (size_t)(s0 + p) * 64 + lane;
+                acc[0] += d[0];
+                acc[1] += d[32];
+            }
             break;
-        }
-        default: {  // w5 for t < 64, b5 for t == 64
-            if (t > 64) return;
-            float acc = 0.f;
-            for (int s = s0; s < s1; ++s) acc += t < 64 ? A.dl[s] * A.a4[(size_t)s * 64 + t] : A.dl[s];
-            P[t < 64 ? kOffW5 + t : kOffB5] = acc;
+        default:  // w5, b5
+            used = 3;
+#pragma unroll 4
+            for (int p = warp; p < cnt; p += kWW) {
+                const float dl = A.dl[s0 + p];
+                const float* a = A.a4 + (size_t)(s0 + p) * 64 + lane;
+                acc[0] = fmaf(dl, a[0], acc[0]);
+                acc[1] = fmaf(dl, a[32], acc[1]);
+                acc[2] += dl;
+            }
             break;
-        }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        if (k < used) red[warp][k * 32 + lane] = acc[k];
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t >= used * 32) return;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWW; ++w) v += red[w][t];
+    const int k = t >> 5;
+    switch (blockIdx.y) {
+        case 0: P[k < 5 ? kOffW1 + lane * 5 + k : kOffB1 + lane] = v; break;
+        case 1: P[kOffB2 + lane] = v; break;
+        case 2: P[kOffB3 + lane] = v; break;
+        case 3: P[kOffB4 + t] = v; break;
+        default:
+            if (k < 2) P[kOffW5 + t] = v;
+            else if (lane == 0) P[kOffB5] = v;
+            break;
     }
 }
 
@@ -314,11 +317,15 @@ struct AdamArgs {
     float lr, beta1, beta2, eps, c1, c2;  // c1 = 1 - beta1^t, c2 = 1 - beta2^t
 };
 
-__global__ void reduce_adam_kernel(const float* part, int chunks, float* grad, float* master, float* m, float* v,
+constexpr int kRedT = 128;
+__global__ void __launch_bounds__(kRedT) reduce_adam_kernel(const float* part, int chunks, float* grad, float* master, float* m, float* v,
                                    float* wq, AdamArgs aa) {
+    dev::pdl_launch();
+    dev::pdl_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= kParams) return;
     float g = 0.f;
+#pragma unroll 8
     for (int c = 0; c < chunks; ++c) g += part[(size_t)c * kParams + p];
     if (grad) grad[p] = g;
     if (!aa.adam) return;
@@ -333,6 +340,8 @@ __global__ void reduce_adam_kernel(const float* part, int chunks, float* grad, f
 
 // Deterministic mean of the per-sample losses (one CTA).
 __global__ void loss_mean_kernel(const float* loss, int n, float* out) {
+    dev::pdl_launch();
+    dev::pdl_wait();
     __shared__ float red[256];
     float acc = 0.f;
     for (int s = threadIdx.x; s < n; s += 256) acc += loss[s];
@@ -894,8 +903,22 @@ constexpr int kMaxSmem = 2 * stage_bytes(kMaxN) + 64;  // the largest launch (N 
 // Where a D element goes. kPlain: out[y * out_chunk + m * out_ld + n]. The
 // weight-gradient layouts write into the parameter vector of chunk y
 // (out = part, out_chunk = kParams): kW2T m = tap * 32 + in, n = out;
-// kW3T m = (tap - 2) * 32 + in, n = out; kW4 m = hidden, n = in.
-enum OutMap { kPlain = 0, kW2T = 1, kW3T = 2, kW4 = 3 };
+// kW3T m = (tap - 2) * 32 + in, n = out; kW4 m = hidden, n = in. The layers'
+// own epilogues (kFwd, kBwd; m = sample, an Epilogue) replace a pass of its own
+// over the layer's outputs after each GEMM.
+enum OutMap { kW2T = 1, kW3T = 2, kW4 = 3, kFwd = 4, kBwd = 5 };
+
+// kFwd: v = ReLU(D + bias[n]), rounded to bf16 when rnd; kBwd: v = act > 0 ?
+// D : 0 (act like f). Into f [samples][ld] at column col + n, and, when given,
+// bf16 copies b (like f) and t [ld][ldt], transposed, whose columns m_valid ..
+// m_valid rounded up to 8 get 0.
+struct Epilogue {
+    const float* bias;
+    const float* act;
+    float* f;
+    uint16_t *b, *t;
+    int ld, ldt, col, rnd;
+};
 
 struct GemmArgs {
     int N;           // columns of D: a multiple of 32, at most 256
@@ -904,8 +927,9 @@ struct GemmArgs {
     int ksplit;      // K per blockIdx.y (a multiple of kKS)
     int m_valid;     // rows of D that are stored
     int map;         // OutMap
-    float* out;
-    size_t out_ld, out_chunk;
+    float* out;      // weight gradients
+    size_t out_chunk;
+    Epilogue ep;
     uint32_t tmem_cols;  // power of two >= max(N, 32)
     int32_t* status;
 };
@@ -948,6 +972,7 @@ __global__ void __launch_bounds__(kNT, 1) gemm_kernel(const __grid_constant__ CU
     const int kend = min(k0 + g.ksplit, g.klen);
     const int nk = kend > k0 ? (kend - k0 + kKS - 1) / kKS : 0;  // stages per pass
     const int total = nk * g.npass;
+    dev::pdl_launch();
     if (tid == 0) {
         for (int i = 0; i < 5; ++i) dev::mbar_init(&bars[i], 1);
         dev::fence_barrier_init();
@@ -967,6 +992,7 @@ __global__ void __launch_bounds__(kNT, 1) gemm_kernel(const __grid_constant__ CU
     inf::fence_before();
     __syncthreads();
     inf::fence_after();
+    dev::pdl_wait();  // operands (and what the epilogue reads) complete
     const uint32_t tm = *tslot;
     // instruction descriptor: bf16 x bf16 -> fp32, both K-major, M = 128
     const uint32_t id = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(g.N >> 3) << 17) | (uint32_t(kTM >> 4) << 24);
@@ -1032,17 +1058,42 @@ __global__ void __launch_bounds__(kNT, 1) gemm_kernel(const __grid_constant__ CU
         for (int c0 = 0; c0 < g.N; c0 += 32) {
             float v[32];
             inf::ld32(tl + c0, v);
-            if (row < g.m_valid) {
-                if (g.map == kPlain) {
-                    float* o = outc + (size_t)row * g.out_ld + c0;
+            if (g.map >= kFwd) {
+                const Epilogue& e = g.ep;
+                const int c = e.col + c0;
+                if (row < g.m_valid) {
+                    const size_t o = (size_t)row * e.ld + c;
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                } else {
+                    for (int j = 0; j < 32; j += 4) {
+                        float* w = v + j;
+                        if (g.map == kFwd) {
+                            const float4 q = *reinterpret_cast<const float4*>(e.bias + c0 + j);
+                            w[0] = fmaxf(w[0] + q.x, 0.f); w[1] = fmaxf(w[1] + q.y, 0.f);
+                            w[2] = fmaxf(w[2] + q.z, 0.f); w[3] = fmaxf(w[3] + q.w, 0.f);
+                            if (e.rnd)
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const int p = out_index(g.map, row, c0 + j);
-                        if (p >= 0) outc[p] = v[j];
+                                for (int k = 0; k < 4; ++k) w[k] = bf16r(w[k]);
+                        } else {
+                            const float4 q = *reinterpret_cast<const float4*>(e.act + o + j);
+                            w[0] = q.x > 0.f ? w[0] : 0.f; w[1] = q.y > 0.f ? w[1] : 0.f;
+                            w[2] = q.z > 0.f ? w[2] : 0.f; w[3] = q.w > 0.f ? w[3] : 0.f;
+                        }
+                        *reinterpret_cast<float4*>(e.f + o + j) = make_float4(w[0], w[1], w[2], w[3]);
+                        if (e.b)
+                            *reinterpret_cast<uint2*>(e.b + o + j) =
+                                make_uint2(bf16_bits(w[0]) | uint32_t(bf16_bits(w[1])) << 16,
+                                           bf16_bits(w[2]) | uint32_t(bf16_bits(w[3])) << 16);
                     }
+                }
+                if (e.t && row < ((g.m_valid + 7) & ~7))
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        e.t[(size_t)(c + j) * e.ldt + row] = row < g.m_valid ? bf16_bits(v[j]) : uint16_t(0);
+            } else if (row < g.m_valid) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    const int p = out_index(g.map, row, c0 + j);
+                    if (p >= 0) outc[p] = v[j];
                 }
             }
         }
@@ -1066,6 +1117,8 @@ struct TrainW {
 constexpr int kTrainWElems = 32 * 160 + 32 * 64 + 64 * 32 + 32 * 64 + 64 * 32 + 224 * 64;
 
 __global__ void pack_train_weights_kernel(const float* wq, TrainW w) {
+    dev::pdl_launch();
+    dev::pdl_wait();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < kTrainWElems; k += gridDim.x * blockDim.x) {
         int e = k;
         if (e < 32 * 160) {
@@ -1164,12 +1217,32 @@ int operand_map(CUtensorMap* m, const uint16_t* base, int rows, int K, size_t pi
     return make_tmap_nd(m, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 3, dims, strides, box);
 }
 
+// Launches a training kernel with programmatic stream serialisation: its
+// launch and prologue overlap the kernel before it (the step is about 16 short
+// launches, one after another).
+template <typename... P, typename... Args>
+int launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const Args&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    CT_LAUNCH_CHECK();
+    return CT_OK;
+}
+
 // D = sum over passes of A_p x B_p^T on the tensor cores (tg::gemm_kernel):
 // M rows of A, N rows of B (a multiple of 32), K = klen split into ksplit
 // per blockIdx.y.
 int tc_gemm(ConfNetHandle* h, const CUtensorMap& a0, const CUtensorMap& b0, const CUtensorMap* a1,
-            const CUtensorMap* b1, int M, int N, int klen, int ksplit, int map, float* out, size_t out_ld,
-            size_t out_chunk, cudaStream_t s) {
+            const CUtensorMap* b1, int M, int N, int klen, int ksplit, int map, const tg::Epilogue& ep,
+            cudaStream_t s) {
     tg::GemmArgs g{};
     g.N = N;
     g.npass = a1 ? 2 : 1;
@@ -1177,15 +1250,14 @@ int tc_gemm(ConfNetHandle* h, const CUtensorMap& a0, const CUtensorMap& b0, cons
     g.ksplit = ksplit;
     g.m_valid = M;
     g.map = map;
-    g.out = out;
-    g.out_ld = out_ld;
-    g.out_chunk = out_chunk;
+    g.out = h->part;
+    g.out_chunk = kParams;
+    g.ep = ep;
     g.tmem_cols = N <= 32 ? 32u : N <= 64 ? 64u : N <= 128 ? 128u : 256u;
     g.status = h->d_status;
     const dim3 grid((M + tg::kTM - 1) / tg::kTM, (klen + ksplit - 1) / ksplit);
-    tg::gemm_kernel<<<grid, tg::kNT, 2 * tg::stage_bytes(N) + 64, s>>>(a0, b0, a1 ? *a1 : a0, b1 ? *b1 : b0, g);
-    CT_LAUNCH_CHECK();
-    return CT_OK;
+    return launch_after(tg::gemm_kernel, grid, dim3(tg::kNT), 2 * tg::stage_bytes(N) + 64, s, a0, b0, a1 ? *a1 : a0,
+                        b1 ? *b1 : b0, g);
 }
 
 // forward (+ backward when labels are given) of n samples on stream s:
@@ -1195,66 +1267,84 @@ int tc_gemm(ConfNetHandle* h, const CUtensorMap& a0, const CUtensorMap& b0, cons
 int run_train_graph(ConfNetHandle* h, const uint8_t* x, const uint8_t* labels, int n, float* scores,
                     cudaStream_t s) {
     const Act& A = h->act;
-    const dim3 b32(32, kSY), b64(64, 8), be(32, 8);
-    const int g32 = (n + kSY - 1) / kSY, g64 = (n + 7) / 8, ge = (n + 7) / 8;
     const int n8 = (n + 7) & ~7;
     const size_t lt = size_t(A.ldt);
+    // the first launch is an ordinary one: it waits for whatever came before
     tg::pack_train_weights_kernel<<<(tg::kTrainWElems + 255) / 256, 256, 0, s>>>(h->wq, h->tw);
-    fwd1_kernel<<<g32, b32, 0, s>>>(x, h->wq, A, n);
     CT_LAUNCH_CHECK();
+    if (int rc = launch_after(fwd1_kernel, dim3((n8 + kSY - 1) / kSY), dim3(32, kSY), 0, s, x, h->wq, A, n)) return rc;
     const int kS = tg::kKS;
     auto ks = [&](int k) { return (k + kS - 1) / kS * kS; };  // whole K in one CTA
+    auto fwd = [&](int bias, float* f, uint16_t* b, uint16_t* t, int ld, int col, int rnd) {
+        return tg::Epilogue{h->wq + bias, nullptr, f, b, t, ld, A.ldt, col, rnd};
+    };
+    auto bwd = [&](const float* act, float* f, uint16_t* b, uint16_t* t, int ld) {
+        return tg::Epilogue{nullptr, act, f, b, t, ld, A.ldt, 0, 0};
+    };
     CUtensorMap ma, mb, ma2, mb2;
     // conv2: position r reads slots 3 r .. 3 r + 4 of a1p (160 contiguous values)
     if (int rc = operand_map(&mb, h->tw.w2f, 32, 160, 160, 32)) return rc;
     for (int r = 0; r < kR; ++r) {
         if (int rc = operand_map(&ma, A.a1p + 96 * r, n, 160, 256, tg::kTM)) return rc;
-        if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 32, 160, ks(160), tg::kPlain, A.d + 32 * r, 64, 0, s))
+        if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 32, 160, ks(160), tg::kFwd,
+                             fwd(kOffB2, A.a2, A.a2b, A.a2t, 64, 32 * r, 1), s))
             return rc;
     }
-    ep_fwd_kernel<<<ge, be, 0, s>>>(A.d, 64, h->wq + kOffB2, 32, 1, A.a2, A.a2b, A.a2t, A.ldt, n);
     // conv3 (taps 2, 3 over both positions) and fc1
     if (int rc = operand_map(&ma, A.a2b, n, 64, 64, tg::kTM)) return rc;
     if (int rc = operand_map(&mb, h->tw.w3f, 32, 64, 64, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 32, 64, ks(64), tg::kPlain, A.d, 32, 0, s)) return rc;
-    ep_fwd_kernel<<<ge, be, 0, s>>>(A.d, 32, h->wq + kOffB3, 32, 1, A.a3, A.a3b, A.a3t, A.ldt, n);
+    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 32, 64, ks(64), tg::kFwd,
+                         fwd(kOffB3, A.a3, A.a3b, A.a3t, 32, 0, 1), s))
+        return rc;
     if (int rc = operand_map(&ma, A.a3b, n, 32, 32, tg::kTM)) return rc;
     if (int rc = operand_map(&mb, h->tw.w4f, 64, 32, 32, 64)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 64, 32, ks(32), tg::kPlain, A.d, 64, 0, s)) return rc;
-    ep_fwd_kernel<<<ge, be, 0, s>>>(A.d, 64, h->wq + kOffB4, 64, 0, A.a4, nullptr, nullptr, A.ldt, n);
-    head_kernel<<<(n + 255) / 256, 256, 0, s>>>(h->wq, A, labels, 1.f / float(n), scores, n);
-    CT_LAUNCH_CHECK();
+    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 64, 32, ks(32), tg::kFwd,
+                         fwd(kOffB4, A.a4, nullptr, nullptr, 64, 0, 0), s))
+        return rc;
+    if (int rc = launch_after(head_kernel, dim3((n8 + kHeadT / 32 - 1) / (kHeadT / 32)), dim3(kHeadT), 0, s, h->wq, A,
+                              labels, 1.f / float(n), scores, n))
+        return rc;
     if (!labels) return CT_OK;
     // data gradients
-    bwd4_kernel<<<g64, b64, 0, s>>>(h->wq, A, n);
     if (int rc = operand_map(&ma, A.dz4b, n, 64, 64, tg::kTM)) return rc;
     if (int rc = operand_map(&mb, h->tw.w4t, 32, 64, 64, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 32, 64, ks(64), tg::kPlain, A.d, 32, 0, s)) return rc;
-    ep_bwd_kernel<<<ge, be, 0, s>>>(A.d, 32, A.a3, A.dz3, A.dz3b, A.dz3t, A.ldt, n);
+    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 32, 64, ks(64), tg::kBwd,
+                         bwd(A.a3, A.dz3, A.dz3b, A.dz3t, 32), s))
+        return rc;
     if (int rc = operand_map(&ma, A.dz3b, n, 32, 32, tg::kTM)) return rc;
     if (int rc = operand_map(&mb, h->tw.w3t, 64, 32, 32, 64)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 64, 32, ks(32), tg::kPlain, A.d, 64, 0, s)) return rc;
-    ep_bwd_kernel<<<ge, be, 0, s>>>(A.d, 64, A.a2, A.dz2, A.dz2b, A.dz2t, A.ldt, n);
+    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 64, 32, ks(32), tg::kBwd,
+                         bwd(A.a2, A.dz2, A.dz2b, A.dz2t, 64), s))
+        return rc;
     if (int rc = operand_map(&ma, A.dz2b, n, 64, 64, tg::kTM)) return rc;
     if (int rc = operand_map(&mb, h->tw.w2t, 224, 64, 64, 224)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 224, 64, ks(64), tg::kPlain, A.d, 224, 0, s)) return rc;
-    ep_bwd_kernel<<<ge, be, 0, s>>>(A.d, 224, A.a1, A.dm1, nullptr, nullptr, A.ldt, n);
+    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 224, 64, ks(64), tg::kBwd,
+                         bwd(A.a1, A.dm1, nullptr, nullptr, 224), s))
+        return rc;
     // weight gradients per chunk of kChunk samples into part[chunk][param]
     // conv2: sum over positions r of a1p slots 3 r .. 3 r + 4 (rows) x dz2 position r
+    const tg::Epilogue none{};
     if (int rc = operand_map(&ma, A.a1pt, 160, n8, lt, tg::kTM)) return rc;
     if (int rc = operand_map(&mb, A.dz2t, 32, n8, lt, 32)) return rc;
     if (int rc = operand_map(&ma2, A.a1pt + 96 * lt, 160, n8, lt, tg::kTM)) return rc;
     if (int rc = operand_map(&mb2, A.dz2t + 32 * lt, 32, n8, lt, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, &ma2, &mb2, 160, 32, n8, kChunk, tg::kW2T, h->part, 0, kParams, s)) return rc;
+    if (int rc = tc_gemm(h, ma, mb, &ma2, &mb2, 160, 32, n8, kChunk, tg::kW2T, none, s)) return rc;
     if (int rc = operand_map(&ma, A.a2t, 64, n8, lt, tg::kTM)) return rc;
     if (int rc = operand_map(&mb, A.dz3t, 32, n8, lt, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, 64, 32, n8, kChunk, tg::kW3T, h->part, 0, kParams, s)) return rc;
+    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, 64, 32, n8, kChunk, tg::kW3T, none, s)) return rc;
     if (int rc = operand_map(&ma, A.dz4t, 64, n8, lt, tg::kTM)) return rc;
     if (int rc = operand_map(&mb, A.a3t, 32, n8, lt, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, 64, 32, n8, kChunk, tg::kW4, h->part, 0, kParams, s)) return rc;
-    wgrad_kernel<<<dim3(chunks_for(n), 5), 256, 0, s>>>(x, A, n, h->part);
-    CT_LAUNCH_CHECK();
-    return CT_OK;
+    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, 64, 32, n8, kChunk, tg::kW4, none, s)) return rc;
+    return launch_after(wgrad_kernel, dim3(chunks_for(n), 5), dim3(32 * kWW), 0, s, x, A, n, h->part);
+}
+
+// Sums the chunks' gradients (and applies them with aa.adam), and the loss.
+int finish_step(ConfNetHandle* h, int n, float* grad, const AdamArgs& aa, float* loss, cudaStream_t s) {
+    if (int rc = launch_after(reduce_adam_kernel, dim3((kParams + kRedT - 1) / kRedT), dim3(kRedT), 0, s, h->part,
+                              chunks_for(n), grad, h->master, h->m, h->v, h->wq, aa))
+        return rc;
+    if (!loss) return CT_OK;
+    return launch_after(loss_mean_kernel, dim3(1), dim3(256), 0, s, h->act.loss, n, loss);
 }
 
 // Packs master weights into the inference image (host side).
@@ -1359,7 +1449,7 @@ int ct_confnet_configure(ct_handle* hh, int32_t device, int32_t max_batch) {
                  o_a2t = take(2 * 64 * ldt), o_a3b = take(2 * 32 * n), o_a3t = take(2 * 32 * ldt),
                  o_dz4b = take(2 * 64 * n), o_dz4t = take(2 * 64 * ldt), o_dz3b = take(2 * 32 * n),
                  o_dz3t = take(2 * 32 * ldt), o_dz2b = take(2 * 64 * n), o_dz2t = take(2 * 64 * ldt),
-                 o_d = take(4 * 224 * n), o_tw = take(2 * tg::kTrainWElems);
+                 o_tw = take(2 * tg::kTrainWElems);
     cudaFree(h->arena);
     h->arena = nullptr;
     if (cudaMalloc(&h->arena, bytes) != cudaSuccess) return fail(CT_ENOMEM, "confidence-net scratch (%zu bytes)", bytes);
@@ -1397,7 +1487,6 @@ int ct_confnet_configure(ct_handle* hh, int32_t device, int32_t max_batch) {
     h->act.dz3t = u16(o_dz3t);
     h->act.dz2b = u16(o_dz2b);
     h->act.dz2t = u16(o_dz2t);
-    h->act.d = reinterpret_cast<float*>(A + o_d);
     h->act.ldt = int(ldt);
     uint16_t* tw = u16(o_tw);
     h->tw.w2f = tw;
@@ -1496,11 +1585,7 @@ int ct_confnet_loss_grad(ct_handle* hh, const uint8_t* samples, const uint8_t* l
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     h->last_stream = s;
     if (int rc = run_train_graph(h, samples, labels, n, nullptr, s)) return rc;
-    reduce_adam_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(h->part, chunks_for(n), grad ? grad : h->grad, h->master,
-                                                            h->m, h->v, h->wq, AdamArgs{0, 0, 0, 0, 0, 1, 1});
-    if (loss) loss_mean_kernel<<<1, 256, 0, s>>>(h->act.loss, n, loss);
-    CT_LAUNCH_CHECK();
-    return CT_OK;
+    return finish_step(h, n, grad ? grad : h->grad, AdamArgs{0, 0, 0, 0, 0, 1, 1}, loss, s);
 }
 
 int ct_confnet_train_step(ct_handle* hh, const uint8_t* samples, const uint8_t* labels, int32_t n, float lr,
@@ -1518,10 +1603,7 @@ int ct_confnet_train_step(ct_handle* hh, const uint8_t* samples, const uint8_t* 
     const float b1 = 0.9f, b2 = 0.999f;
     AdamArgs aa{1, lr, b1, b2, 1e-8f, float(1.0 - std::pow(double(b1), h->steps)),
                 float(1.0 - std::pow(double(b2), h->steps))};
-    reduce_adam_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(h->part, chunks_for(n), h->grad, h->master, h->m, h->v,
-                                                            h->wq, aa);
-    if (loss) loss_mean_kernel<<<1, 256, 0, s>>>(h->act.loss, n, loss);
-    CT_LAUNCH_CHECK();
+    if (int rc = finish_step(h, n, h->grad, aa, loss, s)) return rc;
     h->wimg_dirty = true;
     return CT_OK;
 }
