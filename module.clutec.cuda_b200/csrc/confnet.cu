@@ -139,39 +139,66 @@ struct Act {  // per-sample activations and gradient signals, [n][...]
 constexpr int kQ = 7;   // pooled conv1 positions
 constexpr int kR = 2;   // conv2 positions
 
-constexpr int kSY = 16;  // samples per CTA
+constexpr int kSY = 16;        // warps of a CTA
+constexpr int kSN = 2 * kSY;   // its samples: two a warp
 
-// conv1 (k=5, stride 5) over the 35 central codes, ReLU, bf16; also the
-// bf16 operand copies of the conv2 GEMMs (forward and weight gradient)
+// conv1 (k=5, stride 5) over the 35 central codes, ReLU, bf16, lane = channel;
+// also the bf16 operand copies of the conv2 GEMMs (forward and weight
+// gradient). The transposed copy goes through shared memory so that its rows
+// are written 64 bytes at a time (2 bytes a lane, a row apart, took 28 us for
+// 8192 samples).
 __global__ void __launch_bounds__(32 * kSY) fwd1_kernel(const uint8_t* x, const float* wq, Act A, int n) {
+    __shared__ uint16_t tr[kQ * 32][kSN + 2];
     dev::pdl_launch();
     dev::pdl_wait();
-    __shared__ float xs[kSY][kLen];
-    const int o = threadIdx.x, sl = threadIdx.y, s = blockIdx.x * kSY + sl;
-    for (int k = threadIdx.x; k < kLen; k += 32) xs[sl][k] = s < n ? float(x[(size_t)s * kLen + k]) : 0.f;
-    __syncthreads();
-    if (s >= ((n + 7) & ~7)) return;
-    if (s >= n) {  // transposed columns past n read as 0
-#pragma unroll
-        for (int q = 0; q <= kQ; ++q) A.a1pt[(size_t)(q * 32 + o) * A.ldt + s] = 0;
-        return;
-    }
+    const int o = threadIdx.x;
     float w[5];
 #pragma unroll
     for (int j = 0; j < 5; ++j) w[j] = wq[kOffW1 + o * 5 + j];
     const float b = wq[kOffB1 + o];
-    A.a1p[(size_t)s * 256 + o] = 0;
-    A.a1pt[(size_t)o * A.ldt + s] = 0;
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) {
-        float z = b;
+    for (int k = 0; k < 2; ++k) {
+        const int sl = threadIdx.y + kSY * k, s = blockIdx.x * kSN + sl;
+        if (s >= n) {  // transposed columns past n read as 0
 #pragma unroll
-        for (int j = 0; j < 5; ++j) z = fmaf(w[j], xs[sl][kCropLo + 5 * q + j], z);
-        const float v = bf16r(fmaxf(z, 0.f));
-        A.a1[(size_t)s * 224 + q * 32 + o] = v;
-        const uint16_t vb = bf16_bits(v);
-        A.a1p[(size_t)s * 256 + (q + 1) * 32 + o] = vb;
-        A.a1pt[(size_t)((q + 1) * 32 + o) * A.ldt + s] = vb;
+            for (int q = 0; q < kQ; ++q) tr[q * 32 + o][sl] = 0;
+            continue;
+        }
+        // the 35 codes as 9 words, the same for every lane (kCropLo and kLen
+        // are multiples of 4; x is a device allocation of whole samples)
+        uint32_t c[9];
+        const uint8_t* xs = x + (size_t)s * kLen + kCropLo;
+        const bool words = (reinterpret_cast<uintptr_t>(x) & 3) == 0;
+#pragma unroll
+        for (int i = 0; i < 9; ++i)
+            c[i] = words ? reinterpret_cast<const uint32_t*>(xs)[i]
+                         : xs[4 * i] | uint32_t(xs[4 * i + 1]) << 8 | uint32_t(xs[4 * i + 2]) << 16 |
+                               uint32_t(xs[4 * i + 3]) << 24;
+        A.a1p[(size_t)s * 256 + o] = 0;
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+            float z = b;
+#pragma unroll
+            for (int j = 0; j < 5; ++j) {
+                const int i = 5 * q + j;
+                z = fmaf(w[j], float((c[i >> 2] >> (8 * (i & 3))) & 255u), z);
+            }
+            const float v = bf16r(fmaxf(z, 0.f));
+            A.a1[(size_t)s * 224 + q * 32 + o] = v;
+            const uint16_t vb = bf16_bits(v);
+            A.a1p[(size_t)s * 256 + (q + 1) * 32 + o] = vb;
+            tr[q * 32 + o][sl] = vb;
+        }
+    }
+    __syncthreads();
+    // rows of a1pt: slot 0 is 0, then the 7 positions; 16 lanes a row, two
+    // samples (4 bytes) a lane. ldt is a multiple of 8 and covers n rounded up
+    // to 8.
+    const int s = blockIdx.x * kSN + 2 * (threadIdx.x & 15);
+    if (s >= ((n + 7) & ~7)) return;
+    for (int r = 2 * threadIdx.y + (threadIdx.x >> 4); r < 256; r += 2 * kSY) {
+        const uint32_t v = r < 32 ? 0u : *reinterpret_cast<const uint32_t*>(&tr[r - 32][2 * (threadIdx.x & 15)]);
+        *reinterpret_cast<uint32_t*>(&A.a1pt[(size_t)r * A.ldt + s]) = v;
     }
 }
 
@@ -242,14 +269,28 @@ __global__ void __launch_bounds__(32 * kWW) wgrad_kernel(const uint8_t* x, Act A
             used = 6;
             const float* g0 = A.dm1 + (size_t)s0 * 224 + lane;
             const uint8_t* x0 = x + (size_t)s0 * kLen + kCropLo;
-#pragma unroll 4
-            for (int p = warp; p < cnt * kQ; p += kWW) {
-                const int s = p / kQ, q = p - s * kQ;
-                const float g = g0[p * 32];
-                const uint8_t* xs = x0 + s * kLen + 5 * q;
+            const bool words = (reinterpret_cast<uintptr_t>(x) & 3) == 0;
+#pragma unroll 2
+            for (int s = warp; s < cnt; s += kWW) {  // a sample's 35 codes as 9 words (as fwd1_kernel)
+                float g[kQ];
+                uint32_t c[9];
 #pragma unroll
-                for (int j = 0; j < 5; ++j) acc[j] = fmaf(g, float(xs[j]), acc[j]);
-                acc[5] += g;
+                for (int q = 0; q < kQ; ++q) g[q] = g0[s * 224 + q * 32];
+                const uint8_t* xs = x0 + s * kLen;
+#pragma unroll
+                for (int i = 0; i < 9; ++i)
+                    c[i] = words ? reinterpret_cast<const uint32_t*>(xs)[i]
+                                 : xs[4 * i] | uint32_t(xs[4 * i + 1]) << 8 | uint32_t(xs[4 * i + 2]) << 16 |
+                                       uint32_t(xs[4 * i + 3]) << 24;
+#pragma unroll
+                for (int q = 0; q < kQ; ++q) {
+#pragma unroll
+                    for (int j = 0; j < 5; ++j) {
+                        const int i = 5 * q + j;
+                        acc[j] = fmaf(g[q], float((c[i >> 2] >> (8 * (i & 3))) & 255u), acc[j]);
+                    }
+                    acc[5] += g[q];
+                }
             }
             break;
         }
@@ -921,7 +962,7 @@ struct Epilogue {
 };
 
 struct GemmArgs {
-    int N;           // columns of D: a multiple of 32, at most 256
+    int N;           // columns of D a CTA takes (blockIdx.z-th N rows of B): a multiple of 32, at most 256
     int npass;       // operand pairs accumulated into D (1 or 2)
     int klen;        // K of each pass
     int ksplit;      // K per blockIdx.y (a multiple of kKS)
@@ -967,7 +1008,7 @@ __global__ void __launch_bounds__(kNT, 1) gemm_kernel(const __grid_constant__ CU
     const int SB = stage_bytes(g.N);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * SB);  // full[2], free[2], done
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 5);
-    const int m0 = blockIdx.x * kTM;
+    const int m0 = blockIdx.x * kTM, n0 = blockIdx.z * g.N;
     const int k0 = blockIdx.y * g.ksplit;
     const int kend = min(k0 + g.ksplit, g.klen);
     const int nk = kend > k0 ? (kend - k0 + kKS - 1) / kKS : 0;  // stages per pass
@@ -1012,7 +1053,7 @@ __global__ void __launch_bounds__(kNT, 1) gemm_kernel(const __grid_constant__ CU
 #pragma unroll
                 for (int c = 0; c < kKS / 8; ++c) {
                     dev::tma_load_3d(sa + c * kTM * 16, ma, 0, kk / 8 + c, m0, &bars[s]);
-                    dev::tma_load_3d(sb + c * g.N * 16, mb, 0, kk / 8 + c, 0, &bars[s]);
+                    dev::tma_load_3d(sb + c * g.N * 16, mb, 0, kk / 8 + c, n0, &bars[s]);
                 }
             }
             __syncwarp();
@@ -1060,14 +1101,14 @@ __global__ void __launch_bounds__(kNT, 1) gemm_kernel(const __grid_constant__ CU
             inf::ld32(tl + c0, v);
             if (g.map >= kFwd) {
                 const Epilogue& e = g.ep;
-                const int c = e.col + c0;
+                const int c = e.col + n0 + c0;
                 if (row < g.m_valid) {
                     const size_t o = (size_t)row * e.ld + c;
 #pragma unroll
                     for (int j = 0; j < 32; j += 4) {
                         float* w = v + j;
                         if (g.map == kFwd) {
-                            const float4 q = *reinterpret_cast<const float4*>(e.bias + c0 + j);
+                            const float4 q = *reinterpret_cast<const float4*>(e.bias + n0 + c0 + j);
                             w[0] = fmaxf(w[0] + q.x, 0.f); w[1] = fmaxf(w[1] + q.y, 0.f);
                             w[2] = fmaxf(w[2] + q.z, 0.f); w[3] = fmaxf(w[3] + q.w, 0.f);
                             if (e.rnd)
@@ -1184,6 +1225,11 @@ bool bf16_to_f16_exact(float v, uint16_t* out) {
     return __half2float(h) == v;
 }
 
+struct TrainMaps {
+    int n = 0;  // samples they were made for (0: none)
+    CUtensorMap w2f, w3f, w4f, w4t, w3t, w2t, a1p[2], a2b, a3b, dz4b, dz3b, dz2b, a1pt[2], dz2t[2], a2t, dz3t, dz4t, a3t;
+};
+
 struct ConfNetHandle : ct_handle {
     ConfNetHandle() : ct_handle(Kind::ConfNet) {}
     ~ConfNetHandle() override {
@@ -1197,6 +1243,7 @@ struct ConfNetHandle : ct_handle {
     unsigned char* wimg = nullptr;  // packed inference weights
     tg::TrainW tw{};                // bf16 B operands of the training GEMMs
     Act act{};
+    TrainMaps maps;                 // operand maps of the last step's size (train_maps)
     int steps = 0;
     bool wimg_dirty = true;
     int sms = 148;
@@ -1238,10 +1285,11 @@ int launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaS
 }
 
 // D = sum over passes of A_p x B_p^T on the tensor cores (tg::gemm_kernel):
-// M rows of A, N rows of B (a multiple of 32), K = klen split into ksplit
-// per blockIdx.y.
+// M rows of A, nsplit x N rows of B (N a multiple of 32), K = klen split into
+// ksplit per blockIdx.y. The epilogues take most of a CTA's time here, so wide
+// layers split their columns (224 columns of 8192 samples in 64 CTAs: 26 us).
 int tc_gemm(ConfNetHandle* h, const CUtensorMap& a0, const CUtensorMap& b0, const CUtensorMap* a1,
-            const CUtensorMap* b1, int M, int N, int klen, int ksplit, int map, const tg::Epilogue& ep,
+            const CUtensorMap* b1, int M, int N, int nsplit, int klen, int ksplit, int map, const tg::Epilogue& ep,
             cudaStream_t s) {
     tg::GemmArgs g{};
     g.N = N;
@@ -1255,9 +1303,38 @@ int tc_gemm(ConfNetHandle* h, const CUtensorMap& a0, const CUtensorMap& b0, cons
     g.ep = ep;
     g.tmem_cols = N <= 32 ? 32u : N <= 64 ? 64u : N <= 128 ? 128u : 256u;
     g.status = h->d_status;
-    const dim3 grid((M + tg::kTM - 1) / tg::kTM, (klen + ksplit - 1) / ksplit);
+    const dim3 grid((M + tg::kTM - 1) / tg::kTM, (klen + ksplit - 1) / ksplit, nsplit);
     return launch_after(tg::gemm_kernel, grid, dim3(tg::kNT), 2 * tg::stage_bytes(N) + 64, s, a0, b0, a1 ? *a1 : a0,
                         b1 ? *b1 : b0, g);
+}
+
+// The operand maps of a step of n samples, all over the handle's own scratch:
+// made again only when n changes (20 encodings a step are host time that a
+// step of short launches waits for).
+int train_maps(ConfNetHandle* h, int n) {
+    if (h->maps.n == n) return CT_OK;
+    h->maps.n = 0;
+    TrainMaps& M = h->maps;
+    const Act& A = h->act;
+    const int n8 = (n + 7) & ~7;
+    const size_t lt = size_t(A.ldt);
+    struct One { CUtensorMap* m; const uint16_t* p; int rows, k; size_t pitch; int box; };
+    const One all[] = {
+        {&M.w2f, h->tw.w2f, 32, 160, 160, 32},   {&M.w3f, h->tw.w3f, 32, 64, 64, 32},
+        {&M.w4f, h->tw.w4f, 64, 32, 32, 32},     {&M.w4t, h->tw.w4t, 32, 64, 64, 32},
+        {&M.w3t, h->tw.w3t, 64, 32, 32, 32},     {&M.w2t, h->tw.w2t, 224, 64, 64, 32},
+        {&M.a1p[0], A.a1p, n, 160, 256, tg::kTM}, {&M.a1p[1], A.a1p + 96, n, 160, 256, tg::kTM},
+        {&M.a2b, A.a2b, n, 64, 64, tg::kTM},     {&M.a3b, A.a3b, n, 32, 32, tg::kTM},
+        {&M.dz4b, A.dz4b, n, 64, 64, tg::kTM},   {&M.dz3b, A.dz3b, n, 32, 32, tg::kTM},
+        {&M.dz2b, A.dz2b, n, 64, 64, tg::kTM},
+        {&M.a1pt[0], A.a1pt, 160, n8, lt, tg::kTM}, {&M.a1pt[1], A.a1pt + 96 * lt, 160, n8, lt, tg::kTM},
+        {&M.dz2t[0], A.dz2t, 32, n8, lt, 32},    {&M.dz2t[1], A.dz2t + 32 * lt, 32, n8, lt, 32},
+        {&M.a2t, A.a2t, 64, n8, lt, tg::kTM},    {&M.dz3t, A.dz3t, 32, n8, lt, 32},
+        {&M.dz4t, A.dz4t, 64, n8, lt, tg::kTM},  {&M.a3t, A.a3t, 32, n8, lt, 32}};
+    for (const One& o : all)
+        if (int rc = operand_map(o.m, o.p, o.rows, o.k, o.pitch, o.box)) return rc;
+    M.n = n;
+    return CT_OK;
 }
 
 // forward (+ backward when labels are given) of n samples on stream s:
@@ -1267,74 +1344,49 @@ int tc_gemm(ConfNetHandle* h, const CUtensorMap& a0, const CUtensorMap& b0, cons
 int run_train_graph(ConfNetHandle* h, const uint8_t* x, const uint8_t* labels, int n, float* scores,
                     cudaStream_t s) {
     const Act& A = h->act;
+    if (int rc = train_maps(h, n)) return rc;
+    const TrainMaps& M = h->maps;
     const int n8 = (n + 7) & ~7;
-    const size_t lt = size_t(A.ldt);
     // the first launch is an ordinary one: it waits for whatever came before
     tg::pack_train_weights_kernel<<<(tg::kTrainWElems + 255) / 256, 256, 0, s>>>(h->wq, h->tw);
     CT_LAUNCH_CHECK();
-    if (int rc = launch_after(fwd1_kernel, dim3((n8 + kSY - 1) / kSY), dim3(32, kSY), 0, s, x, h->wq, A, n)) return rc;
-    const int kS = tg::kKS;
-    auto ks = [&](int k) { return (k + kS - 1) / kS * kS; };  // whole K in one CTA
-    auto fwd = [&](int bias, float* f, uint16_t* b, uint16_t* t, int ld, int col, int rnd) {
-        return tg::Epilogue{h->wq + bias, nullptr, f, b, t, ld, A.ldt, col, rnd};
+    if (int rc = launch_after(fwd1_kernel, dim3((n8 + kSN - 1) / kSN), dim3(32, kSY), 0, s, x, h->wq, A, n)) return rc;
+    auto ks = [](int k) { return (k + tg::kKS - 1) / tg::kKS * tg::kKS; };  // whole K in one CTA
+    auto fwd = [&](const CUtensorMap& a, const CUtensorMap& b, int nsplit, int k, const tg::Epilogue& e) {
+        return tc_gemm(h, a, b, nullptr, nullptr, n, 32, nsplit, k, ks(k), tg::kFwd, e, s);
     };
-    auto bwd = [&](const float* act, float* f, uint16_t* b, uint16_t* t, int ld) {
-        return tg::Epilogue{nullptr, act, f, b, t, ld, A.ldt, 0, 0};
+    auto bwd = [&](const CUtensorMap& a, const CUtensorMap& b, int nsplit, int k, const float* act, float* f,
+                   uint16_t* fb, uint16_t* ft) {
+        const tg::Epilogue e{nullptr, act, f, fb, ft, 32 * nsplit, A.ldt, 0, 0};
+        return tc_gemm(h, a, b, nullptr, nullptr, n, 32, nsplit, k, ks(k), tg::kBwd, e, s);
     };
-    CUtensorMap ma, mb, ma2, mb2;
+    auto wgrad = [&](const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap* a1, const CUtensorMap* b1, int m,
+                     int map) {
+        return tc_gemm(h, a, b, a1, b1, m, 32, 1, n8, kChunk, map, tg::Epilogue{}, s);
+    };
+    const float* bias = h->wq;
     // conv2: position r reads slots 3 r .. 3 r + 4 of a1p (160 contiguous values)
-    if (int rc = operand_map(&mb, h->tw.w2f, 32, 160, 160, 32)) return rc;
-    for (int r = 0; r < kR; ++r) {
-        if (int rc = operand_map(&ma, A.a1p + 96 * r, n, 160, 256, tg::kTM)) return rc;
-        if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 32, 160, ks(160), tg::kFwd,
-                             fwd(kOffB2, A.a2, A.a2b, A.a2t, 64, 32 * r, 1), s))
+    for (int r = 0; r < kR; ++r)
+        if (int rc = fwd(M.a1p[r], M.w2f, 1, 160,
+                         {bias + kOffB2, nullptr, A.a2, A.a2b, A.a2t, 64, A.ldt, 32 * r, 1}))
             return rc;
-    }
     // conv3 (taps 2, 3 over both positions) and fc1
-    if (int rc = operand_map(&ma, A.a2b, n, 64, 64, tg::kTM)) return rc;
-    if (int rc = operand_map(&mb, h->tw.w3f, 32, 64, 64, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 32, 64, ks(64), tg::kFwd,
-                         fwd(kOffB3, A.a3, A.a3b, A.a3t, 32, 0, 1), s))
-        return rc;
-    if (int rc = operand_map(&ma, A.a3b, n, 32, 32, tg::kTM)) return rc;
-    if (int rc = operand_map(&mb, h->tw.w4f, 64, 32, 32, 64)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 64, 32, ks(32), tg::kFwd,
-                         fwd(kOffB4, A.a4, nullptr, nullptr, 64, 0, 0), s))
+    if (int rc = fwd(M.a2b, M.w3f, 1, 64, {bias + kOffB3, nullptr, A.a3, A.a3b, A.a3t, 32, A.ldt, 0, 1})) return rc;
+    if (int rc = fwd(M.a3b, M.w4f, 2, 32, {bias + kOffB4, nullptr, A.a4, nullptr, nullptr, 64, A.ldt, 0, 0}))
         return rc;
     if (int rc = launch_after(head_kernel, dim3((n8 + kHeadT / 32 - 1) / (kHeadT / 32)), dim3(kHeadT), 0, s, h->wq, A,
                               labels, 1.f / float(n), scores, n))
         return rc;
     if (!labels) return CT_OK;
     // data gradients
-    if (int rc = operand_map(&ma, A.dz4b, n, 64, 64, tg::kTM)) return rc;
-    if (int rc = operand_map(&mb, h->tw.w4t, 32, 64, 64, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 32, 64, ks(64), tg::kBwd,
-                         bwd(A.a3, A.dz3, A.dz3b, A.dz3t, 32), s))
-        return rc;
-    if (int rc = operand_map(&ma, A.dz3b, n, 32, 32, tg::kTM)) return rc;
-    if (int rc = operand_map(&mb, h->tw.w3t, 64, 32, 32, 64)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 64, 32, ks(32), tg::kBwd,
-                         bwd(A.a2, A.dz2, A.dz2b, A.dz2t, 64), s))
-        return rc;
-    if (int rc = operand_map(&ma, A.dz2b, n, 64, 64, tg::kTM)) return rc;
-    if (int rc = operand_map(&mb, h->tw.w2t, 224, 64, 64, 224)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, n, 224, 64, ks(64), tg::kBwd,
-                         bwd(A.a1, A.dm1, nullptr, nullptr, 224), s))
-        return rc;
+    if (int rc = bwd(M.dz4b, M.w4t, 1, 64, A.a3, A.dz3, A.dz3b, A.dz3t)) return rc;
+    if (int rc = bwd(M.dz3b, M.w3t, 2, 32, A.a2, A.dz2, A.dz2b, A.dz2t)) return rc;
+    if (int rc = bwd(M.dz2b, M.w2t, 7, 64, A.a1, A.dm1, nullptr, nullptr)) return rc;
     // weight gradients per chunk of kChunk samples into part[chunk][param]
     // conv2: sum over positions r of a1p slots 3 r .. 3 r + 4 (rows) x dz2 position r
-    const tg::Epilogue none{};
-    if (int rc = operand_map(&ma, A.a1pt, 160, n8, lt, tg::kTM)) return rc;
-    if (int rc = operand_map(&mb, A.dz2t, 32, n8, lt, 32)) return rc;
-    if (int rc = operand_map(&ma2, A.a1pt + 96 * lt, 160, n8, lt, tg::kTM)) return rc;
-    if (int rc = operand_map(&mb2, A.dz2t + 32 * lt, 32, n8, lt, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, &ma2, &mb2, 160, 32, n8, kChunk, tg::kW2T, none, s)) return rc;
-    if (int rc = operand_map(&ma, A.a2t, 64, n8, lt, tg::kTM)) return rc;
-    if (int rc = operand_map(&mb, A.dz3t, 32, n8, lt, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, 64, 32, n8, kChunk, tg::kW3T, none, s)) return rc;
-    if (int rc = operand_map(&ma, A.dz4t, 64, n8, lt, tg::kTM)) return rc;
-    if (int rc = operand_map(&mb, A.a3t, 32, n8, lt, 32)) return rc;
-    if (int rc = tc_gemm(h, ma, mb, nullptr, nullptr, 64, 32, n8, kChunk, tg::kW4, none, s)) return rc;
+    if (int rc = wgrad(M.a1pt[0], M.dz2t[0], &M.a1pt[1], &M.dz2t[1], 160, tg::kW2T)) return rc;
+    if (int rc = wgrad(M.a2t, M.dz3t, nullptr, nullptr, 64, tg::kW3T)) return rc;
+    if (int rc = wgrad(M.dz4t, M.a3t, nullptr, nullptr, 64, tg::kW4)) return rc;
     return launch_after(wgrad_kernel, dim3(chunks_for(n), 5), dim3(32 * kWW), 0, s, x, A, n, h->part);
 }
 
@@ -1452,6 +1504,7 @@ int ct_confnet_configure(ct_handle* hh, int32_t device, int32_t max_batch) {
                  o_tw = take(2 * tg::kTrainWElems);
     cudaFree(h->arena);
     h->arena = nullptr;
+    h->maps.n = 0;
     if (cudaMalloc(&h->arena, bytes) != cudaSuccess) return fail(CT_ENOMEM, "confidence-net scratch (%zu bytes)", bytes);
     CT_CUDA_TRY(cudaMemset(h->arena, 0, bytes));
     unsigned char* A = h->arena;
