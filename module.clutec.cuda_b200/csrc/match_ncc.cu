@@ -181,24 +181,9 @@ __global__ void __launch_bounds__(kNT, 2)
         dev::fence_barrier_init();
     }
     for (int i = tid; i < a.th * TWO; i += kNT) sKey[i] = 0ull;
-    // Disparity block z covers dz0 = base + z kDPC .. + kDPC - 1. Unguided,
-    // base = 0. Guided, base starts at the low end (rounded down to kDPW) of
-    // the union of the search ranges of the 16 x 16 blocks this tile's
-    // outputs fall in, so a tile whose union is narrow needs one block; the
-    // others, and the warps of a block above the union, do no matching (the
-    // outputs are still written below).
-    int base = 0, ulo = 0, uhi = a.D - 1;
-    if (a.guide) {
-        const int2 u = guide::tile_union(a.guide, a.guide_gw, xs + R, min(xs + R + TWO, a.W) - 1, y0,
-                                         min(y0 + a.th, a.H) - 1, reinterpret_cast<int*>(bar + 1));
-        ulo = u.x;
-        uhi = min(u.y, a.D - 1);
-        if (ulo <= uhi) base = ulo & ~(kDPW - 1);
-    }
-    const int dz0 = base + int(blockIdx.z) * kDPC;
+    const int dz0 = int(blockIdx.z) * kDPC;
     const int dw = dz0 + warp * kDPW;
     const bool warp_active = dw < a.D;
-    const bool searches = ulo <= uhi && dw <= uhi && dw + kDPW - 1 >= ulo;
     const int ab = xs & ~15;
     const int am = (xs - a.dmin - dz0 - (kDPC - 1)) & ~15;
     __syncthreads();
@@ -221,7 +206,7 @@ __global__ void __launch_bounds__(kNT, 2)
 #pragma unroll
         for (int c = 0; c < kCPT; ++c) V[j][c] = 0;
 
-    if (warp_active && searches && !aborted) {
+    if (warp_active && !aborted) {
         for (int i = 0; i < NR; ++i) {
             {
                 const uint8_t* rb = sB + i * kBW + bo;
@@ -341,16 +326,10 @@ __global__ void __launch_bounds__(kNT, 2)
                 sxc[c] = a.Sx[o];
                 fvxc[c] = __int2float_rn(a.Vx[o]);
                 tc[c] = a.Tx[o];
-                // searched disparities dw + j: j in [jlo, jhi] (guide range,
-                // match column x - dmin - d - R >= 0)
-                int glo = 0, ghi = a.D - 1;
-                if (a.guide && colok) {
-                    const uint32_t g = __ldg(&a.guide[(size_t)(y / kGuideBlock) * a.guide_gw + x / kGuideBlock]);
-                    glo = int(g & 0xFFFFu);
-                    ghi = min(int(g >> 16), a.D - 1);
-                }
-                const int jlo = max(glo - dw, 0), jhi = min(min(ghi, x - a.dmin - R) - dw, kDPW - 1);
-                const uint32_t smask = (colok && jlo <= jhi) ? ((2u << jhi) - (1u << jlo)) : 0u;
+                // searched disparities dw + j: j <= jhi (match column
+                // x - dmin - d - R >= 0)
+                const int jhi = min(min(a.D - 1, x - a.dmin - R) - dw, kDPW - 1);
+                const uint32_t smask = (colok && jhi >= 0) ? ((2u << jhi) - 1u) : 0u;
                 float val[kDPW];
                 float emax = -INFINITY;
 #pragma unroll
@@ -437,6 +416,7 @@ __global__ void __launch_bounds__(kNT, 2)
 }  // namespace ct
 
 #include "ncc_tc.cuh"
+#include "ncc_guided.cuh"
 
 namespace ct {
 namespace {
@@ -498,7 +478,14 @@ int launch_ncc(NccHandle* h, const ct_image* disp, const ct_image* score, const 
                                           static_cast<const uint8_t*>(Rr->ptr), Rr->pitch_bytes, W, H, h->stats,
                                           h->stats + N, h->stats + 4 * N, h->stats + 2 * N, h->stats + 3 * N);
     CT_LAUNCH_CHECK();
-    if (!init && h->tensor_cores) {
+    if (init) {
+        ncc_guided_kernel<R><<<dim3(a.guide_gw, (H + kGuideBlock - 1) / kGuideBlock), gd::kThreads, 0, s>>>(
+            static_cast<const uint8_t*>(L->ptr), L->pitch_bytes, static_cast<const uint8_t*>(Rr->ptr),
+            Rr->pitch_bytes, a);
+        CT_LAUNCH_CHECK();
+        return gate_launch(disp, score, L, 0, 2 * R + 1, h->grad_thresh, s);  // EvalGrad (NCC.cu:388-413)
+    }
+    if (h->tensor_cores) {
         static bool attr_tc = false;
         if (!attr_tc) {
             CT_CUDA_TRY(cudaFuncSetAttribute(ncc_tc_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
