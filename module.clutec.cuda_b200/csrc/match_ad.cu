@@ -31,23 +31,20 @@ namespace ad {
 constexpr int kCPT = 4, kTWV = 128, kDPC = 64;
 constexpr int kPairs = kDPC / 2;         // disparity pairs per CTA (two disparities per 32-bit register)
 // Disparities per warp DPW (4: 16 warps, 8: 8 warps per CTA; the kernel is
-// instantiated for both): warps, threads, pairs per thread, match columns a
-// thread reads per row.
+// instantiated for both): warps, threads, pairs per thread.
 __host__ __device__ constexpr int nt_of(int dpw) { return kDPC / dpw * 32; }
 constexpr int kBW = kTWV + 16;        // staged base columns
 constexpr int kMWs = kTWV + kDPC + 16; // staged match columns (208)
 constexpr int kRing = 7;              // AW: rows of S kept
 constexpr int kRingW = kTWV + 8;      // AW: padded ring row (4 words each side)
 
-// Per-pixel costs are formed two disparities at a time in the 16-bit halves
-// of a register as max(b + 256 - m, m + 256 - b) = |b - m| + 256 (no borrow
-// crosses the halves); the 256 cancels in the running sums' add/subtract
-// pairs, so every box sum carries (2r+1)^2 * 256 on top of the SAD (at most
-// 81 * 511 = 41391 for 9x9: the 16-bit cost field never reaches 0xFFFF, the
-// "no disparity" marker). The winner's cost in a key is biased by that much.
-constexpr uint32_t kAbsBias = 0x01000100u;
-__host__ __device__ constexpr int box_bias(int R) { return (2 * R + 1) * (2 * R + 1) * 256; }
-static_assert(81 * 511 < 0xFFFF, "biased 9x9 box sums fit the 16-bit cost field");
+// Per-pixel costs are formed four disparities at a time as the bytes of a
+// register (one packed absolute difference, one ALU instruction) and split
+// into the 16-bit halves of two registers for the running sums (a 9x9 sum is
+// at most 81 * 255 = 20655, so the 16-bit cost field never reaches 0xFFFF, the
+// "no disparity" marker). Forming them in 16-bit halves,
+// max(b + 256 - m, m + 256 - b), took six instructions for four.
+static_assert(81 * 255 < 0xFFFF, "9x9 box sums fit the 16-bit cost field");
 
 __host__ __device__ constexpr int ext_of(int R, bool aw) { return aw ? 2 * R : R; }
 __host__ __device__ constexpr int two_of(int R, bool aw) { return kTWV - 2 * ext_of(R, aw); }
@@ -115,7 +112,7 @@ __device__ __forceinline__ void hsum(const uint32_t (&V)[kCPT], uint32_t (&C)[kC
 template <int R, bool AW, int DIR, bool G, int DPW>  // G: guided (AW only)
 __global__ void __launch_bounds__(nt_of(DPW), 1)
     ad_match_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmM, Args a) {
-    constexpr int kDPW = DPW, kNW = kDPC / DPW, kNT = nt_of(DPW), kNP = DPW / 2, kMC = kCPT + DPW - 1;
+    constexpr int kDPW = DPW, kNW = kDPC / DPW, kNT = nt_of(DPW), kNP = DPW / 2;
     static_assert(kNW * kNP == kPairs, "pairs per CTA");
     constexpr int EXT = ext_of(R, AW);
     constexpr int TWO = two_of(R, AW);
@@ -180,29 +177,34 @@ __global__ void __launch_bounds__(nt_of(DPW), 1)
 #pragma unroll
     for (int p = 0; p < kNP; ++p) dlo[p] = uint32_t(dw + 2 * p);
 
-    auto row_pairs = [&](int i, uint32_t (&P)[kCPT][kNP]) {
+    // |b - m| of strip row i: register (c, g) holds the warp's disparities
+    // 4g .. 4g + 3 of column c in its bytes (right-to-left; left-to-right the
+    // match columns run against the disparities, register (c, g) holds
+    // kDPW - 1 - 4g .. kDPW - 4 - 4g). The match bytes are read as the words
+    // around them (at most 3 bytes before; the last word ends within the
+    // staged row: its first byte is at most 199 of 208) and shifted into place.
+    constexpr int kNG = kDPW / 4;
+    const int ms = 8 * (mo & 3);  // the same for the whole CTA
+    auto row_diffs = [&](int i, uint32_t (&P)[kCPT][kNG]) {
         const uint8_t* rb = sB + i * kBW + bo;
-        const uint8_t* rm = sM + i * kMWs + mo;
-        uint32_t b2[kCPT], m2[kMC - 1];
+        const uint32_t* rm = reinterpret_cast<const uint32_t*>(sM + i * kMWs + (mo & ~3));
+        uint32_t w[kNG + 2], m[kNG + 1];
 #pragma unroll
-        for (int c = 0; c < kCPT; ++c) b2[c] = uint32_t(rb[c]) * 0x10001u;  // b in both halves
-        // match pixel pairs: the low half is disparity 2p of the pair, the
-        // high half 2p + 1 (left-to-right: columns k0, k0 - 1; right-to-left:
-        // k0, k0 + 1)
-        {
-            uint32_t m[kMC];
+        for (int k = 0; k < kNG + 2; ++k) w[k] = rm[k];
 #pragma unroll
-            for (int k = 0; k < kMC; ++k) m[k] = rm[k];
+        for (int k = 0; k < kNG + 1; ++k) m[k] = __funnelshift_r(w[k], w[k + 1], ms);
 #pragma unroll
-            for (int k = 0; k < kMC - 1; ++k) m2[k] = DIR == 0 ? m[k + 1] + (m[k] << 16) : m[k] + (m[k + 1] << 16);
+        for (int c = 0; c < kCPT; ++c) {
+            const uint32_t b4 = uint32_t(rb[c]) * 0x01010101u;
+#pragma unroll
+            for (int g = 0; g < kNG; ++g)
+                P[c][g] = __vabsdiffu4(b4, c == 0 ? m[g] : __funnelshift_r(m[g], m[g + 1], 8 * c));
         }
-#pragma unroll
-        for (int c = 0; c < kCPT; ++c)
-#pragma unroll
-            for (int p = 0; p < kNP; ++p) {
-                const uint32_t mp = m2[DIR == 0 ? c - 2 * p + kDPW - 2 : c + 2 * p];
-                P[c][p] = __vmaxu2(b2[c] + kAbsBias - mp, mp + kAbsBias - b2[c]);  // |b - m| + 256 per half
-            }
+    };
+    // pair p's differences (disparity 2p in the low half, 2p + 1 in the high)
+    auto pair = [&](const uint32_t (&P)[kNG], int p) {
+        return DIR == 0 ? __byte_perm(P[kNG - 1 - p / 2], 0u, p & 1 ? 0x4041 : 0x4243)
+                        : __byte_perm(P[p / 2], 0u, p & 1 ? 0x4342 : 0x4140);
     };
 
     uint32_t V[kNP][kCPT];  // [pair][column]
@@ -213,20 +215,20 @@ __global__ void __launch_bounds__(nt_of(DPW), 1)
 
     if (warp_active) {
         for (int i = 0; i < NR; ++i) {
-            uint32_t Pn[kCPT][kNP];
-            row_pairs(i, Pn);
+            uint32_t Pn[kCPT][kNG];
+            row_diffs(i, Pn);
             if (i >= 2 * R + 1) {
-                uint32_t Po[kCPT][kNP];
-                row_pairs(i - 2 * R - 1, Po);
+                uint32_t Po[kCPT][kNG];
+                row_diffs(i - 2 * R - 1, Po);
 #pragma unroll
                 for (int c = 0; c < kCPT; ++c)
 #pragma unroll
-                    for (int p = 0; p < kNP; ++p) V[p][c] = V[p][c] + Pn[c][p] - Po[c][p];
+                    for (int p = 0; p < kNP; ++p) V[p][c] = V[p][c] + pair(Pn[c], p) - pair(Po[c], p);
             } else {
 #pragma unroll
                 for (int c = 0; c < kCPT; ++c)
 #pragma unroll
-                    for (int p = 0; p < kNP; ++p) V[p][c] += Pn[c][p];
+                    for (int p = 0; p < kNP; ++p) V[p][c] += pair(Pn[c], p);
             }
             if (i < 2 * R) continue;
             // S (box sums) of strip row i - R, all 4 pairs
@@ -342,13 +344,15 @@ __global__ void ad_finalize_kernel(uint32_t* keys, int W, int H, int ext, void* 
 // base view's 28 rows x 64 columns around the tile and the match view's rows
 // over the band of columns the tile's winners reach (at most 21 16-byte
 // chunks for D <= 256), then
-// each thread forms the 133 cells of its plus-shaped 13 x 13 neighbourhood
-// with both disparities in the two 16-bit halves (|b - m| + 256, as in the
-// matcher) and sums the five windows from partial column sums.
+// each thread sums the five windows of its plus-shaped 13 x 13 neighbourhood
+// (133 cells a disparity): per row the 13 (or the 7 central) pixels are words
+// shifted into place, four cells a packed absolute difference, and a window's
+// share of the row two or three dot products with a byte mask.
 constexpr int kSpX = 32, kSpTY = 8, kSpQ = 2, kSpY = kSpTY * kSpQ;  // 32 x 16 pixels, 2 rows per thread
 constexpr int kSpRows = kSpY + 12;
 constexpr int kSpLCols = 64;                         // base columns x0 - 16 .. x0 + 47 (16-byte chunks)
-constexpr int kSpRCols = 21 * 16;                    // match band rounded out to 16-byte chunks
+constexpr int kSpRCols = 22 * 16;                    // match band rounded out to 16-byte chunks, one more for
+                                                     // the words read around a thread's last bytes
 
 __global__ void __launch_bounds__(kSpX * kSpTY) aw_subpixel_kernel(uint32_t* keys, int W, int H, int D, int dmin,
                                                                  const uint8_t* L, size_t pl, const uint8_t* Rm,
@@ -439,43 +443,64 @@ __global__ void __launch_bounds__(kSpX * kSpTY) aw_subpixel_kernel(uint32_t* key
         if (!need[q]) continue;
         const int ty = threadIdx.y + kSpTY * q, y = y0 + ty;
         const int e = dmin + int(key[q] & 0xFFFFu);
-        // cell (r, k): row y - 6 + r, column x - 6 + k; base pixel sL[ty + r][tx + 10 + k];
-        // match pixel of disparity e -/+ 1 at band column base + k + 2 / base + k
+        // Row r of the neighbourhood is image row y - 6 + r, byte k column
+        // x - 6 + k: base pixel sL[ty + r][tx + 10 + k], match pixel of
+        // disparity e + 1 at band column base + k, of e - 1 two further.
         const int base = x - e - 7 - rs;
-        auto cell = [&](int r, int k) {
-            const uint32_t b2 = uint32_t(sL[ty + r][tx + 10 + k]) * 0x10001u;
-            const uint32_t m2 = uint32_t(sR[ty + r][base + k + 2]) + (uint32_t(sR[ty + r][base + k]) << 16);
-            return __vmaxu2(b2 + kAbsBias - m2, m2 + kAbsBias - b2);  // (|b - m-| + 256) | (|b - m+| + 256) << 16
+        // d[0], d[1]: |b - m| of disparities e - 1, e + 1 for the bytes k0 ..
+        // k0 + 4 N - 1 of row r, of which k0 .. k0 + 4 N - 4 are used
+        auto diffs = [&](int r, int k0, auto& d) {
+            constexpr int N = sizeof(d[0]) / 4;
+            const int lo = tx + 10 + k0, mo = base + k0, ls = 8 * (lo & 3), ms = 8 * (mo & 3);
+            const uint32_t* pl32 = reinterpret_cast<const uint32_t*>(&sL[ty + r][lo & ~3]);
+            const uint32_t* pm32 = reinterpret_cast<const uint32_t*>(&sR[ty + r][mo & ~3]);
+            uint32_t wl[N + 1], wm[N + 2], m[N + 1];
+#pragma unroll
+            for (int k = 0; k <= N; ++k) wl[k] = pl32[k];
+#pragma unroll
+            for (int k = 0; k <= N; ++k) wm[k] = pm32[k];
+            wm[N + 1] = 0;
+#pragma unroll
+            for (int k = 0; k <= N; ++k) m[k] = __funnelshift_r(wm[k], wm[k + 1], ms);
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const uint32_t b = __funnelshift_r(wl[k], wl[k + 1], ls);
+                d[0][k] = __vabsdiffu4(b, __funnelshift_r(m[k], m[k + 1], 16));
+                d[1][k] = __vabsdiffu4(b, m[k]);
+            }
         };
-        // partial column sums: top rows 0-2, middle 3-5, centre 6, lower 7-9, bottom 10-12
-        uint32_t mid[13], sl = 0, sc = 0, sr = 0, su = 0, sd = 0;
+        // window sums: left, right, and the central columns of rows 0-2, 3-5, 6, 7-9, 10-12
+        uint32_t sl[2] = {0, 0}, sr[2] = {0, 0}, sc[2][5] = {};
 #pragma unroll
-        for (int k = 0; k < 13; ++k) {
-            uint32_t a = 0, m = cell(6, k), c = 0;
+        for (int r = 0; r < 13; ++r) {
+            const int part = r < 3 ? 0 : r < 6 ? 1 : r == 6 ? 2 : r < 10 ? 3 : 4;
+            if (part == 0 || part == 4) {
+                uint32_t d[2][2];
+                diffs(r, 3, d);
 #pragma unroll
-            for (int r = 3; r < 6; ++r) a += cell(r, k);
+                for (int j = 0; j < 2; ++j)
+                    sc[j][part] = __dp4a(d[j][0], 0x01010101u, __dp4a(d[j][1], 0x00010101u, sc[j][part]));
+            } else {
+                uint32_t d[2][4];
+                diffs(r, 0, d);
 #pragma unroll
-            for (int r = 7; r < 10; ++r) c += cell(r, k);
-            mid[k] = a + m + c;
-            if (k >= 3 && k <= 9) {
-                uint32_t t = 0, b = 0;
-#pragma unroll
-                for (int r = 0; r < 3; ++r) t += cell(r, k);
-#pragma unroll
-                for (int r = 10; r < 13; ++r) b += cell(r, k);
-                su += t + a + m;
-                sd += m + c + b;
-                sc += mid[k];
+                for (int j = 0; j < 2; ++j) {
+                    sl[j] = __dp4a(d[j][0], 0x01010101u, __dp4a(d[j][1], 0x00010101u, sl[j]));
+                    sr[j] = __dp4a(d[j][1], 0x01010000u, __dp4a(d[j][2], 0x01010101u, __dp4a(d[j][3], 1u, sr[j])));
+                    sc[j][part] = __dp4a(d[j][0], 0x01000000u,
+                                         __dp4a(d[j][1], 0x01010101u, __dp4a(d[j][2], 0x00000101u, sc[j][part])));
+                }
             }
         }
+        int cost[2];
 #pragma unroll
-        for (int k = 0; k < 7; ++k) {
-            sl += mid[k];
-            sr += mid[k + 6];
+        for (int j = 0; j < 2; ++j) {
+            const uint32_t mid = sc[j][1] + sc[j][2] + sc[j][3];
+            const uint32_t up = sc[j][0] + sc[j][1] + sc[j][2], down = sc[j][2] + sc[j][3] + sc[j][4];
+            cost[j] = int(min(min(mid, min(sl[j], sr[j])), min(up, down)));
         }
-        const uint32_t mn = __vminu2(__vminu2(__vminu2(sc, sl), __vminu2(sr, su)), sd);
-        const int cm = int(mn & 0xFFFFu) - box_bias(3), cp = int(mn >> 16) - box_bias(3);
-        const int c0 = int(key[q] >> 16) - box_bias(3);  // the winner's 7x7 AW cost (keys carry the box bias)
+        const int cm = cost[0], cp = cost[1];
+        const int c0 = int(key[q] >> 16);  // the winner's AW cost
         float sp = float(e);
         const int den = cm - 2 * c0 + cp;
         if (den > 0) sp = __fadd_rn(float(e), __fdiv_rn(float(cm - cp), float(2 * den)));
