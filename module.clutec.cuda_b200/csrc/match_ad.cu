@@ -9,9 +9,9 @@
 // (th + 2*ext rows of the base view, 128 + 16 columns; of the match view,
 // 192 + 16 columns) are staged in shared memory by two 2D TMA loads. Each
 // thread walks the strip downwards keeping vertical running sums of |B - M|
-// for 4 columns x 8 disparities packed as 16-bit pairs; the row leaving the
-// window is recomputed from the staged pixels (cheaper than a register ring
-// for a 1-byte cost). The horizontal pass takes r halo columns from the
+// for 4 columns x 4 or 8 disparities packed as 16-bit pairs; the row leaving
+// the window is kept in registers or formed again from the staged pixels
+// (kKeepRows). The horizontal pass takes r halo columns from the
 // neighbouring lanes by shuffles (AlgoArraySum_W32H16::SumCache's two passes,
 // Kernel.Algo.ArraySum_W32H16.h:163-200).
 // The AW variant stores each row of 7x7 box sums S in a 7-row shared-memory
@@ -109,11 +109,21 @@ __device__ __forceinline__ void hsum(const uint32_t (&V)[kCPT], uint32_t (&C)[kC
     }
 }
 
+// Whether a thread keeps the differences of the rows in its window (registers,
+// 2R + 1 rows of DPW words) or forms those of the leaving row again from the
+// staged pixels. The adaptive windows and the small SAD windows keep them
+// (1920x1080, 240 disparities: AW 480 -> 437 us, SAD 3x3 278 -> 269, 5x5 298
+// -> 294); the 7x7 and 9x9 SAD kernels run two CTAs an SM with 48 registers
+// and lose that (300 -> 318, 302 -> 331).
+template <int R, bool AW>
+constexpr bool kKeepRows = AW || R <= 2;
+
 template <int R, bool AW, int DIR, bool G, int DPW>  // G: guided (AW only)
 __global__ void __launch_bounds__(nt_of(DPW), 1)
     ad_match_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmM, Args a) {
     constexpr int kDPW = DPW, kNW = kDPC / DPW, kNT = nt_of(DPW), kNP = DPW / 2;
     static_assert(kNW * kNP == kPairs, "pairs per CTA");
+    constexpr bool KEEP = kKeepRows<R, AW>;
     constexpr int EXT = ext_of(R, AW);
     constexpr int TWO = two_of(R, AW);
     extern __shared__ __align__(128) unsigned char smem[];
@@ -213,24 +223,38 @@ __global__ void __launch_bounds__(nt_of(DPW), 1)
 #pragma unroll
         for (int c = 0; c < kCPT; ++c) V[p][c] = 0;
 
+    // The differences of the rows in the window, by row index mod 2R + 1: the
+    // row loop is unrolled by that, so that every index is static.
+    constexpr int kU = KEEP ? 2 * R + 1 : 1;
+    uint32_t kept[kU][kCPT][kNG] = {};
+
     if (warp_active) {
-        for (int i = 0; i < NR; ++i) {
+        auto row = [&](const int i, const int u) {
             uint32_t Pn[kCPT][kNG];
             row_diffs(i, Pn);
-            if (i >= 2 * R + 1) {
-                uint32_t Po[kCPT][kNG];
-                row_diffs(i - 2 * R - 1, Po);
+            auto update = [&](const uint32_t (&Po)[kCPT][kNG]) {
 #pragma unroll
                 for (int c = 0; c < kCPT; ++c)
 #pragma unroll
                     for (int p = 0; p < kNP; ++p) V[p][c] = V[p][c] + pair(Pn[c], p) - pair(Po[c], p);
+            };
+            if constexpr (KEEP) {
+                update(kept[u]);  // (0 in the first window)
+#pragma unroll
+                for (int c = 0; c < kCPT; ++c)
+#pragma unroll
+                    for (int g = 0; g < kNG; ++g) kept[u][c][g] = Pn[c][g];
+            } else if (i >= 2 * R + 1) {
+                uint32_t Po[kCPT][kNG];
+                row_diffs(i - 2 * R - 1, Po);
+                update(Po);
             } else {
 #pragma unroll
                 for (int c = 0; c < kCPT; ++c)
 #pragma unroll
                     for (int p = 0; p < kNP; ++p) V[p][c] += pair(Pn[c], p);
             }
-            if (i < 2 * R) continue;
+            if (i < 2 * R) return;
             // S (box sums) of strip row i - R, all 4 pairs
             uint32_t S[kNP][kCPT];
 #pragma unroll
@@ -244,18 +268,20 @@ __global__ void __launch_bounds__(nt_of(DPW), 1)
 #pragma unroll
                     for (int c = 0; c < kCPT; ++c) A[p][c] = S[p][c];
             } else {
-                // S row index since the first S row: s = i - 2R; ring slot s % 7
+                // S row index since the first S row: s = i - 2R; ring slot
+                // s % 7 (u = i % 7)
+                static_assert(!AW || (KEEP && kU == kRing), "ring slots by u");
                 const int s = i - 2 * R;
-                uint32_t* slot = ring + size_t(s % kRing) * kNW * kNP * kRingW;
+                uint32_t* slot = ring + size_t((u + kRing - 2 * R) % kRing) * kNW * kNP * kRingW;
 #pragma unroll
                 for (int p = 0; p < kNP; ++p)
                     *reinterpret_cast<uint4*>(slot + (warp * kNP + p) * kRingW + 4 + 4 * lane) =
                         make_uint4(S[p][0], S[p][1], S[p][2], S[p][3]);
                 __syncwarp();
-                if (s < 2 * R) continue;  // need S rows s - 3 and s - 6
+                if (s < 2 * R) return;  // need S rows s - 3 and s - 6
                 oy = s - 2 * R;
-                const uint32_t* mid = ring + size_t((s - R) % kRing) * kNW * kNP * kRingW;
-                const uint32_t* top = ring + size_t((s - 2 * R) % kRing) * kNW * kNP * kRingW;
+                const uint32_t* mid = ring + size_t((u + 2 * kRing - 3 * R) % kRing) * kNW * kNP * kRingW;
+                const uint32_t* top = ring + size_t((u + 2 * kRing - 4 * R) % kRing) * kNW * kNP * kRingW;
 #pragma unroll
                 for (int p = 0; p < kNP; ++p) {
                     const uint32_t* rm = mid + (warp * kNP + p) * kRingW + 4 * lane;  // padded index of col 4L-4
@@ -273,7 +299,7 @@ __global__ void __launch_bounds__(nt_of(DPW), 1)
                     }
                 }
             }
-            if (oy < 0 || oy >= a.th) continue;
+            if (oy < 0 || oy >= a.th) return;
 #pragma unroll
             for (int c = 0; c < kCPT; ++c) {
                 const int v = 4 * lane + c;
@@ -303,9 +329,12 @@ __global__ void __launch_bounds__(nt_of(DPW), 1)
                 }
                 atomicMin(&sKey[oy * TWO + v - EXT], best);
             }
+        };
+        for (int i = 0; i < NR; i += kU) {
+#pragma unroll
+            for (int u = 0; u < kU; ++u)
+                if (i + u < NR) row(i + u, u);
         }
-    } else if (AW) {
-        // inactive warps still own ring slices nobody reads; nothing to do
     }
     __syncthreads();
     const bool direct = !AW && gridDim.z == 1;
@@ -544,9 +573,10 @@ int set_attr() {
 // Disparities per warp: 4 (16 warps per CTA) for the adaptive windows and
 // the SAD windows from 7x7 up, which are bound by instruction latency at one
 // CTA per SM; 8 for the smaller SAD windows, where loading each base pixel
-// for 8 disparities saves more than the extra warps hide (measured: AW
-// 2560x1440 1.162 -> 1.025 ms and SAD 9x9 640x480 0.0266 -> 0.0245 ms with 4;
-// SAD 5x5 1920x1080 0.1833 ms with 8 against 0.1933 with 4).
+// for 8 disparities saves more than the extra warps hide (measured when the
+// costs were formed two at a time: AW 2560x1440 1.162 -> 1.025 ms and SAD 9x9
+// 640x480 0.0266 -> 0.0245 ms with 4; SAD 5x5 1920x1080 0.1833 ms with 8
+// against 0.1933 with 4).
 template <int R, bool AW>
 constexpr int dpw_for() { return (AW || R >= 3) ? 4 : 8; }
 
