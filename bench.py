@@ -18,9 +18,11 @@ counts pixel x disparity evaluations: 2 directions x W x H x D per step.
               variant (copies in line with the matching on one stream).
   roofline    the dominant kernel (the fused matching pass: each 5x5 Hamming
               cost evaluated once, both directions' winners) timed with CUDA
-              events on its stream, against the POPC-pipe bound (2 POPC per
-              cost) measured live on this GPU by ct_probe_pipe_rates; also the
-              one-direction kernel of process() alone.
+              events on its stream, against the nominal dense FP4 tensor rate
+              (the window sums are FP4 MMAs: 1280 operations per cost); also
+              the one-direction kernel of process() alone, and both as
+              multiples of the POPC-pipe bound (2 POPC per cost) measured live
+              by ct_probe_pipe_rates, which the CUDA-core kernel had.
   cpu_baseline  the CPU restatement (OpenMP, all host threads) on the same
               pair, rank 0 only.
 
@@ -528,11 +530,10 @@ def run_ours(args):
     clock_hz = (clocks["sm_mhz"] or rates["sm_clock_mhz"]) * 1e6
     popc_peak = rates["popc_per_clk_sm"] * sms * clock_hz          # POPC ops / s
     units_launch = W_ * H_ * D_
-    # the fused pass evaluates each 5x5 Hamming cost C(x, d) once (2 POPC)
-    # and decides both directions' winners from it
+    # the matching pass evaluates each 5x5 Hamming cost C(x, d) once and decides
+    # both directions' winners from it; 2 POPC a cost on the CUDA cores
     achieved_popc = 2.0 * units_launch / (fused_ms * 1e-3)
     single_popc = 2.0 * units_launch / (match_ms * 1e-3)           # one direction alone, 2 POPC per unit
-    int_peak = rates["iadd3_per_clk_sm"] * sms * clock_hz
     launches = 3  # census of both views, the fused matching pass, the right-view map + cross-check
 
     out = {
@@ -549,25 +550,23 @@ def run_ours(args):
                 "serial": {"value": round(e2e, 1), "ms_per_step": round(e2e_ms, 4),
                            "api": "ct_bm_census_process_lr with the copies in line on one stream, "
                                   "L2 flushed before every step"}},
-        "roofline": {"bound": "popc", "achieved": round(achieved_popc / 1e12, 4),
-                     "peak": round(popc_peak / 1e12, 4), "unit": "Tpopc/s",
-                     "frac": round(achieved_popc / popc_peak, 4),
+        "roofline": {"bound": "tensor_fp4", "achieved": round(FP4_OPS_PER_COST * units_launch / (fused_ms * 1e-3) / 1e12, 2),
+                     "peak": FP4_PEAK_TFLOPS, "unit": "TFLOP/s",
+                     "frac": round(FP4_OPS_PER_COST * units_launch / (fused_ms * 1e-3) / 1e12 / FP4_PEAK_TFLOPS, 4),
                      "traffic": traffic_from_profile(),
-                     "kernel": "census_match_kernel<0,4,false,true> (the fused pass: 5x5 Hamming costs of "
-                               "1920x1080x128 evaluated once, left-to-right and right-to-left winners; timed as "
+                     "kernel": "census_tc_kernel (the matching pass: 5x5 Hamming costs of 1920x1080x128 as FP4 "
+                               "MMAs, left-to-right and right-to-left winners from one accumulator; timed as "
                                "process_lr(lr, rl) minus the census transform of both views)",
                      "kernel_ms": round(fused_ms, 4), "census_transform_ms": round(census_ms, 4),
-                     "algorithmic_per_unit": "2 POPC per cost C(x, d), one cost per pixel x disparity for both "
-                                             "directions (+ ~9 INT per direction's winner-take-all)",
-                     "frac_per_direction_units": round(2 * achieved_popc / popc_peak, 4),
-                     "frac_per_direction_units_note": "2 W H D direction units per step (the metric's units) "
-                                                      "x 2 POPC each against the same peak",
-                     "single_direction": {"kernel": "census_match_kernel<0,4> (left-to-right alone, process())",
+                     "algorithmic_per_unit": "per cost C(x, d) an entering and a leaving window row of 5 x 64 "
+                                             "multiply-adds = 1280 operations, one cost per pixel x disparity for "
+                                             "both directions",
+                     "popc_equivalent_frac": round(achieved_popc / popc_peak, 4),
+                     "single_direction": {"kernel": "census_tc_kernel (left-to-right alone, process())",
                                           "kernel_ms": round(match_ms, 4),
-                                          "frac": round(single_popc / popc_peak, 4),
-                                          "int_frac_at_9_ops": round(9.0 * units_launch / (match_ms * 1e-3)
-                                                                     / int_peak, 4)},
-                     "peak_source": "ct_probe_pipe_rates measured in this run (POPC/clk/SM x SMs x median SM clock)",
+                                          "popc_equivalent_frac": round(single_popc / popc_peak, 4)},
+                     "peak_source": "nominal dense FP4 (no measured FP4 rate); popc_equivalent: 2 POPC per cost "
+                                    "against ct_probe_pipe_rates x SMs x median SM clock",
                      "pipe_rates_per_clk_sm": {k: round(v, 2) for k, v in rates.items()
                                                if k.endswith("per_clk_sm")}},
         "gpu_launches": launches * args.steps,
@@ -761,17 +760,16 @@ def batch_shapes(n=64, seed=4):
 #   ncc1080: product + 4 box add/sub (5 INT) + normalisation and argmax
 #            (~10 FP32/INT) = 15 lane operations at the issue rate
 #            (128 per SM per clock: 4 schedulers x 32 lanes)
-#   batch64: as the census headline, 2 POPC (64-bit Hamming) per direction
-#            unit; the fused pass evaluates each cost once for both
-#            directions, so frac counts direction units and frac_costs_once
-#            the costs it evaluates
+#   batch64: as the census headline, FP4 MMAs (1280 operations per cost, one
+#            cost for two direction units) against the nominal dense rate
 #   compat1080: the reference's per-disparity NCC (BlockMatcherNCC.cu:218-271:
 #            the cross mean, the test mean and mean square, the test
 #            standard deviation, the normalised and quantised score: 3
 #            divisions, a square root and ~10 other FP32 operations) + the
 #            window sum (5) + the scan update (~8) = 30 lane operations
+FP4_OPS_PER_COST, FP4_PEAK_TFLOPS = 1280, 9000.0  # per cost: 2 rows x 5 x 64 multiply-adds; nominal dense
 ROOF = {"sad640": ("int", 8, "iadd3_per_clk_sm"), "aw1440": ("int", 13, "iadd3_per_clk_sm"),
-        "ncc1080": ("issue", 15, None), "batch64": ("popc", 2, "popc_per_clk_sm"),
+        "ncc1080": ("issue", 15, None), "batch64": ("tensor_fp4", FP4_OPS_PER_COST / 2, None),
         "compat1080": ("issue", 30, None)}
 
 
@@ -779,12 +777,17 @@ def pipe_roofline(kind, ops_per_unit, rate_key, units_per_s, rates, sm_mhz):
     """Integer / issue roofline of a matcher: achieved operations per second
     (units/s x algorithmic ops per unit) against the pipe peak measured on
     this GPU by ct_probe_pipe_rates (per SM per clock x SMs x SM clock)."""
+    if kind == "tensor_fp4":
+        ach = units_per_s * ops_per_unit / 1e12
+        return {"bound": kind, "achieved": round(ach, 2), "peak": FP4_PEAK_TFLOPS, "unit": "TFLOP/s",
+                "frac": round(ach / FP4_PEAK_TFLOPS, 4), "traffic": None,
+                "algorithmic_per_unit": f"{ops_per_unit:g} FP4 operations", "peak_source": "nominal dense FP4"}
     clock_hz = (sm_mhz or rates["sm_clock_mhz"]) * 1e6
     per_clk = 128.0 if rate_key is None else rates[rate_key]
     peak = per_clk * rates["sm_count"] * clock_hz
     ach = units_per_s * ops_per_unit
     return {"bound": kind, "achieved": round(ach / 1e12, 4), "peak": round(peak / 1e12, 4),
-            "unit": {"int": "Tintop/s", "popc": "Tpopc/s", "issue": "Tlaneop/s"}[kind],
+            "unit": {"int": "Tintop/s", "issue": "Tlaneop/s"}[kind],
             "frac": round(ach / peak, 4), "traffic": None, "algorithmic_per_unit": f"{ops_per_unit} {kind} ops",
             "peak_source": ("ct_probe_pipe_rates measured in this run" if rate_key else
                             "issue limit 128 lane-ops/clk/SM") + " x SMs x median SM clock"}
@@ -1072,11 +1075,8 @@ def workload_line(wl, args, ct, dev, stream, flush_buf, world, rank, local, rate
         kind, ops, key = ROOF[wl]
         out_line["roofline"] = pipe_roofline(kind, ops, key, units / (ms * 1e-3), rates, clocks.get("sm_mhz"))
         out_line["roofline"]["note"] = "whole call timed (all its launches)"
-        if wl == "batch64":  # one fused pass per pair decides both directions
-            rf = out_line["roofline"]
-            rf["frac_costs_once"] = round(rf["frac"] / 2, 4)
-            rf["note"] += ("; one fused matching pass per pair evaluates each cost once for both directions: "
-                           "frac counts the metric's direction units (2 per cost), frac_costs_once the costs")
+        if wl == "batch64":
+            out_line["roofline"]["note"] += "; one matching pass per pair evaluates each cost once for both directions"
     if rank != 0:
         return None
     out_line["parity_rank0"] = bool(check_fn())
