@@ -262,8 +262,14 @@ __device__ __forceinline__ float halve(float lo, float hi, bool upper, int mask)
 // Hand-overs to the MMA warp by hardware barriers, which answer in tens of
 // cycles (an mbarrier takes about 200 beside the MMAs' operand reads, longer
 // than the MMAs that wait in the tensor core's queue last): the accumulator of
-// tile t read (barriers 3, 4), staged row r (5-8; the staging warps are at most
-// 2 rows ahead). Every warp keeps taking part when one of its waits gave up.
+// tile t read (barriers 3, 4), staged row r (5-12 in turn). A phase ends with
+// its last arrival, whoever that is, so nobody may arrive for row r + kRowBars
+// before the MMA warp has joined row r: the staging warps write kSlots rows
+// without waiting for anything, and row k >= kSlots once the MMAs of step k - 7
+// are complete, which the MMA warp issued after it joined row k - 3.
+// Every warp keeps taking part when one of its waits gave up.
+constexpr int kRowBars = 8;
+static_assert(kRowBars >= kSlots && 5 + kRowBars <= 16, "staged rows come round to a barrier after the MMA warp has joined it");
 template <int ID, int N>
 __device__ __forceinline__ void bar_arrive() {
     asm volatile("barrier.cta.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
@@ -275,20 +281,10 @@ __device__ __forceinline__ void bar_sync() {
 __device__ __forceinline__ void read_arrive(int t) { t == 0 ? bar_arrive<3, kTileT + 32>() : bar_arrive<4, kTileT + 32>(); }
 __device__ __forceinline__ void read_sync(int t) { t == 0 ? bar_sync<3, kTileT + 32>() : bar_sync<4, kTileT + 32>(); }
 __device__ __forceinline__ void row_arrive(int r) {
-    switch (r & 3) {
-        case 0: bar_arrive<5, kRowT + 32>(); break;
-        case 1: bar_arrive<6, kRowT + 32>(); break;
-        case 2: bar_arrive<7, kRowT + 32>(); break;
-        default: bar_arrive<8, kRowT + 32>();
-    }
+    asm volatile("barrier.cta.arrive %0, %1;" ::"r"(5 + (r & (kRowBars - 1))), "n"(kRowT + 32) : "memory");
 }
 __device__ __forceinline__ void row_sync(int r) {
-    switch (r & 3) {
-        case 0: bar_sync<5, kRowT + 32>(); break;
-        case 1: bar_sync<6, kRowT + 32>(); break;
-        case 2: bar_sync<7, kRowT + 32>(); break;
-        default: bar_sync<8, kRowT + 32>();
-    }
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(5 + (r & (kRowBars - 1))), "n"(kRowT + 32) : "memory");
 }
 // One tile's maxima warps (barriers 1, 2).
 __device__ __forceinline__ void tile_sync(int t) { t == 0 ? bar_sync<1, kTileT>() : bar_sync<2, kTileT>(); }
