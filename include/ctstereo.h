@@ -711,6 +711,12 @@ int ct_probe_pipe_rates(int32_t device, ct_pipe_rates* out);
  * as it would for a tile that never arrived; the kernel returns normally and
  * the context stays usable. The handle must be configured. */
 int ct_handle_test_wait_timeout(ct_handle* h, uint32_t poll_limit, ct_stream stream);
+/* The same for the census matcher's tensor-core pass, whose warps wait for one
+ * another: the waits of this handle's calls give up after poll_limit polls of at
+ * most 20 us (0 .. 65536; 65536, about a second, is the normal limit). A call
+ * whose waits gave up ends in order, sets CT_ETIMEOUT and leaves its maps
+ * unspecified; later calls are not affected. A census matcher or batch handle. */
+int ct_handle_test_wait_limit(ct_handle* h, uint32_t poll_limit);
 
 #ifdef __cplusplus
 }

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kCheckT) check_batch_kernel(const PairDev* pai
 }
 
 __global__ void __launch_bounds__(ctc::kNT, 1)
-    match_batch_kernel(const PairDev* pairs, int n, int total_items, unsigned* queue, int32_t* status) {
+    match_batch_kernel(const PairDev* pairs, int n, int total_items, unsigned* queue, uint32_t polls, int32_t* status) {
     constexpr int NT = ctc::kNT;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ int s_item;
@@ -184,6 +184,7 @@ __global__ void __launch_bounds__(ctc::kNT, 1)
         a.key_pitch = P.rl_pitch;
         a.tag = kTag;
         a.status = status;
+        a.polls = polls;
         if (!ctc::run_tile(c, a, local % P.tiles_x, by)) break;  // status already set; the CTA takes no more work
     }
     ctc::cta_end(c);
@@ -301,7 +302,7 @@ int enqueue(BatchHandle* h, Staging& st, bool record, cudaStream_t s) {
     census_batch_kernel<<<h->total_census, census::kNT, 0, s>>>(h->d_pairs, h->n, h->d_maps, h->d_status);
     CT_LAUNCH_CHECK();
     match_batch_kernel<<<std::min(h->sms, h->total_match), ctc::kNT, ctc::kSmemBytes, s>>>(
-        h->d_pairs, h->n, h->total_match, h->d_queue, h->d_status);
+        h->d_pairs, h->n, h->total_match, h->d_queue, h->wait_polls, h->d_status);
     CT_LAUNCH_CHECK();
     check_batch_kernel<<<h->total_rows, kCheckT, 0, s>>>(h->d_pairs, h->n);
     CT_LAUNCH_CHECK();

@@ -297,6 +297,7 @@ int census_process_tc(BmCensusHandle* h, const ct_image* lr, const ct_image* dis
     a.key_pitch = cm::rl_pitch_words(a.W);
     a.tag = tag;
     a.status = h->d_status;
+    a.polls = h->wait_polls;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(h->tc.tiles_x, (a.H + a.th - 1) / a.th);
     cfg.blockDim = dim3(ctc::kNT);

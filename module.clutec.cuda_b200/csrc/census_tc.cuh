@@ -80,7 +80,7 @@ constexpr int kKeyN = 256;              // right keys of a quarter's row (kNMax,
 constexpr int kOffKeyL = kSlots * kSlotBytes;               // kRowsL x 2 tiles x 2 warps of a quarter x kM keys
 constexpr int kOffKeyR = kOffKeyL + kRowsL * 4 * kM * 4;    // 2 tiles x kRowsR x 4 quarters x kNMax keys
 constexpr int kOffBar = kOffKeyR + 2 * kRowsR * 4 * kKeyN * 4;
-constexpr int kBars = 8 + kRowsL;  // ready, merged
+constexpr int kBars = 8 + kRowsL + 1;  // ready, merged, drained
 constexpr int kOffMisc = kOffBar + kBars * 8;
 constexpr int kSmemBytes = kOffMisc + 32;
 static_assert(kOffKeyL % 16 == 0 && kOffBar % 8 == 0 && kSmemBytes <= 227 * 1024, "shared memory");
@@ -100,6 +100,7 @@ struct Args {
     size_t key_pitch;   // words
     uint32_t tag;       // the call's tag: bids are tag | 23 bits that grow with the key (cm::MaxKeys)
     int32_t* status;
+    uint32_t polls;     // limit of every wait (kPolls; less in tests)
 };
 
 struct Shape {
@@ -187,21 +188,19 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
 }
 // Waits for phase `parity` of `bar`, suspended for up to 20 us a poll (waiting
 // warps that poll more often take the maxima's issue slots), for `polls` polls.
-// Returns the polls for the next wait: the same (about a second), or 0 once a
-// wait gave up.
+// Returns the polls for the warp's next wait: the same (about a second), or 0
+// once a wait gave up.
 constexpr uint32_t kPolls = 1u << 16;
 __device__ __forceinline__ uint32_t wait(uint64_t* bar, uint32_t parity, uint32_t polls) {
     const uint32_t addr = dev::smem_u32(bar);
-    for (uint32_t i = 0; i < polls; ++i) {
-        uint32_t done;
+    uint32_t done = 0;
+    for (uint32_t i = 0; i < polls && !done; ++i)
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done)
             : "r"(addr), "r"(parity), "r"(20000u)
             : "memory");
-        if (done) return polls;
-    }
-    return 0;
+    return __all_sync(0xffffffffu, done) ? polls : 0;
 }
 __device__ __forceinline__ void arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dev::smem_u32(bar)) : "memory");
@@ -267,7 +266,11 @@ __device__ __forceinline__ float halve(float lo, float hi, bool upper, int mask)
 // before the MMA warp has joined row r: the staging warps write kSlots rows
 // without waiting for anything, and row k >= kSlots once the MMAs of step k - 7
 // are complete, which the MMA warp issued after it joined row k - 3.
-// Every warp keeps taking part when one of its waits gave up.
+// A warp whose wait gave up (about a second without an answer) keeps taking part
+// in every hand-over, so that the MMA warp, which waits on nothing else, comes
+// to its end and the CTA can report: it reads, stages and writes nothing more,
+// and arrives for a row once the MMA warp has passed the hand-over that the wait
+// stood behind (Cta::passed).
 constexpr int kRowBars = 8;
 static_assert(kRowBars >= kSlots && 5 + kRowBars <= 16, "staged rows come round to a barrier after the MMA warp has joined it");
 template <int ID, int N>
@@ -295,13 +298,15 @@ struct Cta {
     unsigned char* smem;
     uint64_t* ready;   // [2 tiles][4] window sums of a row complete (commit and the MMA warp's arrival), rows in turn
     uint64_t* merged;  // [kRowsL] tile 0's keys of a row written (kTileWarps arrivals; pairs that share left pixels)
-    uint32_t* misc;    // TMEM address
+    uint64_t* drained; // MMAs complete after a wait gave up
+    uint32_t* misc;    // TMEM address; rows that the MMA warp has begun, per tile
     uint32_t steps0, steps1, merges;  // rows done by tile 0, by tile 1, with merged
     uint32_t tmem;
     __device__ explicit Cta(unsigned char* raw)
         : smem(raw),
           ready(reinterpret_cast<uint64_t*>(raw + kOffBar)),
           merged(ready + 8),
+          drained(merged + kRowsL),
           misc(reinterpret_cast<uint32_t*>(raw + kOffMisc)),
           steps0(0),
           steps1(0),
@@ -311,8 +316,20 @@ struct Cta {
     // Row s of the tile: its barrier, and the wait for it (nobody waits more
     // than 2 rows behind the MMAs, so 4 barriers leave the phase unambiguous).
     __device__ uint64_t* ready_bar(int t, int s) const { return &ready[4 * t + (step(t, s) & 3)]; }
+    // After it, the MMA warp has passed the hand-overs before the row's MMAs,
+    // also when the wait gave up.
     __device__ uint32_t wait_ready(int t, int s, uint32_t polls) const {
-        return wait(ready_bar(t, s), (step(t, s) >> 2) & 1, polls);
+        polls = wait(ready_bar(t, s), (step(t, s) >> 2) & 1, polls);
+        if (polls == 0) passed(t, s);
+        return polls;
+    }
+    __device__ void begin(int t, int s) const { *static_cast<volatile uint32_t*>(misc + 1 + t) = step(t, s) + 1; }
+    // Waits until the MMA warp has begun the row: it waits only for the other
+    // warps' arrivals, each about a second away at most (the limit is about 20).
+    __device__ void passed(int t, int s) const {
+        const volatile uint32_t* begun = misc + 1 + t;
+        for (uint32_t i = 0; i < (1u << 20) && int32_t(*begun - step(t, s)) <= 0; ++i) __nanosleep(20000);
+        __syncwarp();
     }
 };
 
@@ -323,6 +340,8 @@ __device__ __forceinline__ void cta_begin(Cta& c) {
     if (tid == 0) {
         for (int i = 0; i < 8; ++i) dev::mbar_init(&c.ready[i], 2);
         for (int i = 0; i < kRowsL; ++i) dev::mbar_init(&c.merged[i], kTileWarps);
+        dev::mbar_init(c.drained, 1);
+        c.misc[1] = c.misc[2] = 0;
         dev::fence_barrier_init();
     }
     if (warp == 0) {
@@ -374,7 +393,7 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
     const int nrows = rows + 2 * kR;          // staged rows
     const int tiles = x0 + a.lstep < a.W ? 2 : 1;  // a strip's last pair may have one tile only
     const bool share = a.lstep == 0;               // the tiles have the same left pixels
-    uint32_t polls = kPolls;
+    uint32_t polls = a.polls;
 
     if (warp >= (kMaxT + kRowT) / 32) {
         // ---- MMAs
@@ -392,7 +411,10 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
         // holds about 4 MMAs, and a second commit would wait for it to drain.
         auto step = [&](int t, int s) {
             read_sync(t);
-            if (lane == 0) arrive(c.ready_bar(t, s));  // hands on what the reads' arrivals ordered
+            if (lane == 0) {
+                c.begin(t, s);
+                arrive(c.ready_bar(t, s));  // hands on what the reads' arrivals ordered
+            }
             __syncwarp();
             fence_after();
             if (s == 0) {
@@ -441,6 +463,10 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
         auto stage = [&](int k, const uint64_t (&v)[kRowPx]) {
             // row k - 8 left both windows with the last tile's step k - 7
             if (k >= kSlots) polls = c.wait_ready(tiles - 1, k - kSlots + 1, polls);
+            if (polls == 0) {  // (MMAs may still read the slot)
+                row_arrive(k);
+                return;
+            }
             unsigned char* s = c.smem + (k % kSlots) * kSlotBytes;
 #pragma unroll
             for (int j = 0; j < kRowPx; ++j) {
@@ -562,6 +588,11 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
         float* const put_kr = keyR + q * kKeyN;
         for (int s = 0; s < rows; ++s) {
             polls = c.wait_ready(t, s, polls);
+            if (polls == 0) {  // hand-overs only
+                read_arrive(t);
+                if (share && t == 0 && lane == 0) arrive(&c.merged[(c.merges + uint32_t(s)) & (kRowsL - 1)]);
+                continue;
+            }
             fence_after();
             __syncwarp();
             float rm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -659,13 +690,14 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
                 __syncwarp();
                 if (lane == 0) arrive(&c.merged[(c.merges + uint32_t(s)) & (kRowsL - 1)]);
             }
-            if (s >= 2) put(s - 2, k0, k1);
+            if (s >= 2 && polls) put(s - 2, k0, k1);
         }
         // the last two rows
         tile_sync(t);
         for (int r = max(rows - 2, 0); r < rows; ++r) {
             float k0 = 0.0f, k1 = 0.0f;
             wait_merged(r);
+            if (polls == 0) break;
             take(r, k0, k1);
             put(r, k0, k1);
         }
@@ -674,7 +706,14 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
     if (tiles == 2) c.steps1 += uint32_t(rows);
     if (share) c.merges += uint32_t(rows);
     const bool failed = __syncthreads_or(polls == 0);
-    if (failed && tid == 0) dev::report(a.status, CT_ETIMEOUT);
+    if (failed) {
+        if (tid == 0) dev::report(a.status, CT_ETIMEOUT);
+        if (warp == kNT / 32 - 1) {  // the MMA warp: none may be in flight when the CTA ends
+            commit(c.drained);
+            wait(c.drained, 0, kPolls);
+        }
+        __syncthreads();
+    }
     return !failed;
 }
 

@@ -63,6 +63,7 @@ struct Handle {
     int32_t* d_status = nullptr;   // one int32 in device memory
     cudaStream_t last_stream = nullptr;
     float grad_thresh = 0.0f;      // gradient gate of the SAD / NCC / AW matchers (0: off)
+    uint32_t wait_polls = 1u << 16;  // census tensor-core pass: limit of its waits (less in tests)
     explicit Handle(Kind k) : kind(k) {}
     virtual ~Handle();
     int init_status();             // allocates d_status on the current device

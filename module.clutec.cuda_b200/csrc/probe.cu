@@ -130,6 +130,17 @@ extern "C" int ct_probe_pipe_rates(int32_t device, ct_pipe_rates* out) {
     return CT_OK;
 }
 
+extern "C" int ct_handle_test_wait_limit(ct_handle* h, uint32_t poll_limit) {
+    using namespace ct;
+    clear_error();
+    if (!h) return fail(CT_EINVAL, "null handle");
+    if (h->kind != Kind::BmCensus && h->kind != Kind::Batch)
+        return fail(CT_ESTATE, "not a census matcher or batch handle");
+    if (poll_limit > (1u << 16)) return fail(CT_EINVAL, "poll_limit must be 0..65536");
+    h->wait_polls = poll_limit;
+    return CT_OK;
+}
+
 extern "C" int ct_handle_test_wait_timeout(ct_handle* h, uint32_t poll_limit, ct_stream stream) {
     using namespace ct;
     clear_error();

@@ -172,6 +172,7 @@ def _declare(L: C.CDLL) -> None:
         "ct_bm_compat_configure": [H, C.c_int32, fmt, P(ct_compat_params)],
         "ct_bm_compat_process": [H, img, img, img, C.c_void_p],
         "ct_handle_test_wait_timeout": [H, C.c_uint32, C.c_void_p],
+        "ct_handle_test_wait_limit": [H, C.c_uint32],
         "ct_curves_pitch": [C.c_int32, P(C.c_size_t)],
         "ct_bm_census_process_curves": [H, img, P(ct_curves), img, img, C.c_void_p],
         "ct_confnet_create": [P(H)],
@@ -322,6 +323,11 @@ class _Driver:
         """ct_handle_test_wait_timeout: a bounded device wait that nothing
         completes gives up and sets this handle's status to CT_ETIMEOUT."""
         check(lib().ct_handle_test_wait_timeout(self._h, poll_limit, _stream(stream)))
+
+    def test_wait_limit(self, poll_limit: int):
+        """ct_handle_test_wait_limit: poll limit of the waits inside the census
+        tensor-core pass of this handle's calls (65536: normal)."""
+        check(lib().ct_handle_test_wait_limit(self._h, poll_limit))
 
 
 def _fmt(width, height, type_=CT_PIX_U8):

@@ -44,10 +44,17 @@ class Wrong(AssertionError):
 
 class Model:
     """One strip of a tile pair. Actors are generators; what they yield is a
-    condition to wait for."""
+    condition to wait for, or with a second value True a wait that may give up
+    (it then yields False). `give_up` is the chance of that for each time such a
+    wait is looked at in vain; `stuck`: the tensor core completes nothing.
+    `passed`: after it gave up a warp goes on when the MMA warp has begun the row
+    (False: at once)."""
 
-    def __init__(self, rng, rows, tiles, row_bars):
+    def __init__(self, rng, rows, tiles, row_bars, give_up=0.0, stuck=False, passed=True):
         self.rng, self.rows, self.tiles = rng, rows, tiles
+        self.give_up, self.stuck, self.passed = give_up, stuck, passed
+        self.failed = False                # some wait gave up
+        self.begun = [0] * tiles           # rows the MMA warp has begun
         self.row = [Barrier(ROW_WARPS + 1) for _ in range(row_bars)]
         self.read = [Barrier(TILE_WARPS + 1) for _ in range(tiles)]
         self.staged = [[-1] * ROW_WARPS for _ in range(SLOTS)]  # row held by a slot, each warp's part
@@ -68,6 +75,9 @@ class Model:
             yield self.sync(self.row[k % len(self.row)])
             for t in range(self.tiles):
                 yield self.sync(self.read[t])
+                self.begun[t] = s + 1
+                if self.failed:
+                    continue
                 if any(r < s for r in self.reads[t]):
                     raise Wrong(f"tile {t} row {s}: accumulator not read")
                 for r in (range(WIN) if s == 0 else (k, s - 1)):
@@ -75,7 +85,18 @@ class Model:
                         raise Wrong(f"tile {t} row {s}: row {r} not staged")
                 self.issued.append((t, s))
 
+    def ready(self, t, s, ok):
+        """wait_ready: row s of tile t complete; after a give-up, begun."""
+        ok = ok and (yield lambda: self.done[t] > s, True)
+        if not ok:
+            self.failed = True
+            if self.passed:
+                yield lambda: self.begun[t] > s
+        return ok
+
     def tensor_core(self):
+        if self.stuck:
+            return
         for _ in range(self.rows * self.tiles):
             yield lambda: self.issued
             t, s = self.issued.pop(0)
@@ -83,19 +104,23 @@ class Model:
             self.done[t] = s + 1
 
     def staging_warp(self, w):
+        ok = True
         for k in range(self.rows + WIN - 1):
             if k >= SLOTS:
-                yield lambda: self.done[self.tiles - 1] > k - SLOTS + 1
+                ok = yield from self.ready(self.tiles - 1, k - SLOTS + 1, ok)
             yield lambda: True
-            self.staged[k % SLOTS][w] = k
+            if ok:
+                self.staged[k % SLOTS][w] = k
             self.row[k % len(self.row)].arrive()
 
     def maxima_warp(self, t, w):
         yield lambda: True
         self.read[t].arrive()
+        ok = True
         for s in range(self.rows):
-            yield lambda: self.done[t] > s
-            self.reads[t][w] = s + 1
+            ok = yield from self.ready(t, s, ok)
+            if ok:
+                self.reads[t][w] = s + 1
             self.read[t].arrive()
 
     def run(self):
@@ -103,15 +128,24 @@ class Model:
         actors += [self.maxima_warp(t, w) for t in range(self.tiles) for w in range(TILE_WARPS)]
         # an actor's share of the steps: some are held back for long
         share = [10.0 ** self.rng.uniform(-4, 0) for _ in actors]
-        waits = [next(a) for a in actors]
+        unpack = lambda y: y if isinstance(y, tuple) else (y, False)  # noqa: E731
+        waits = [next(a, None) for a in actors]
         while True:
-            ready = [i for i, c in enumerate(waits) if c is not None and c()]
+            live = [(i, *unpack(c)) for i, c in enumerate(waits) if c is not None]
+            ready = [(i, c, b) for i, c, b in live if c() or (b and self.give_up)]
             if not ready:
                 break
-            i = self.rng.choices(ready, [share[i] for i in ready])[0]
-            waits[i] = next(actors[i], None)
-        if any(c is not None for c in waits):
-            raise Wrong(f"stalled: actors {[i for i, c in enumerate(waits) if c is not None]}")
+            i, c, b = self.rng.choices(ready, [share[i] for i, _, _ in ready])[0]
+            ok = bool(c())
+            if not ok and self.rng.random() >= self.give_up:
+                continue
+            try:
+                waits[i] = actors[i].send(ok)
+            except StopIteration:
+                waits[i] = None
+        left = [i for i, c in enumerate(waits) if c is not None and not (i == 1 and self.failed)]
+        if left:
+            raise Wrong(f"stalled: actors {left}")
 
 
 def _schedules(n, **kw):
@@ -129,3 +163,18 @@ def test_the_model_finds_barriers_that_come_round_too_early():
     barriers let a row's phase end without it."""
     with pytest.raises(Wrong):
         _schedules(400, row_bars=SLOTS // 2)
+
+
+@pytest.mark.parametrize("stuck", [False, True])
+def test_a_warp_that_gave_up_keeps_the_hand_overs_in_step(stuck):
+    """Whichever waits give up, and if the tensor core never answers, every warp
+    comes to its end (where the CTA reports the failure)."""
+    assert re.search(r"if \(polls == 0\) passed\(t, s\);", SRC)  # the rule as modelled
+    _schedules(400, row_bars=_row_bars(), give_up=0.05, stuck=stuck)
+
+
+def test_the_model_finds_arrivals_that_run_ahead_after_a_give_up():
+    """Arrivals that nothing holds back end phases without the MMA warp, which
+    then waits for good."""
+    with pytest.raises(Wrong):
+        _schedules(400, row_bars=_row_bars(), give_up=0.05, stuck=True, passed=False)
