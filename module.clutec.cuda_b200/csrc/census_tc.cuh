@@ -189,17 +189,19 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
 // Waits for phase `parity` of `bar`, suspended for up to 20 us a poll (waiting
 // warps that poll more often take the maxima's issue slots), for `polls` polls.
 // Returns the polls for the warp's next wait: the same (about a second), or 0
-// once a wait gave up.
+// once a wait gave up; the warp's lanes agree, and meet, in the vote.
 constexpr uint32_t kPolls = 1u << 16;
 __device__ __forceinline__ uint32_t wait(uint64_t* bar, uint32_t parity, uint32_t polls) {
     const uint32_t addr = dev::smem_u32(bar);
     uint32_t done = 0;
-    for (uint32_t i = 0; i < polls && !done; ++i)
+    for (uint32_t i = 0; i < polls; ++i) {
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done)
             : "r"(addr), "r"(parity), "r"(20000u)
             : "memory");
+        if (done) break;
+    }
     return __all_sync(0xffffffffu, done) ? polls : 0;
 }
 __device__ __forceinline__ void arrive(uint64_t* bar) {
@@ -411,10 +413,7 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
         // holds about 4 MMAs, and a second commit would wait for it to drain.
         auto step = [&](int t, int s) {
             read_sync(t);
-            if (lane == 0) {
-                c.begin(t, s);
-                arrive(c.ready_bar(t, s));  // hands on what the reads' arrivals ordered
-            }
+            if (lane == 0) arrive(c.ready_bar(t, s));  // hands on what the reads' arrivals ordered
             __syncwarp();
             fence_after();
             if (s == 0) {
@@ -424,6 +423,7 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
                 row_mmas(t, s - 1, id_sub);
             }
             commit(c.ready_bar(t, s));
+            if (lane == 0) c.begin(t, s);  // (after the MMAs: before them it cost 1%)
         };
         for (int k = 0; k < kWin - 1; ++k) row_sync(k);
         for (int s = 0; s < rows; ++s) {
@@ -594,7 +594,6 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
                 continue;
             }
             fence_after();
-            __syncwarp();
             float rm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             // Maxima of a piece: along the rows into rm, along the columns
             // (over the thread's 4 rows) into w.
@@ -690,7 +689,7 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
                 __syncwarp();
                 if (lane == 0) arrive(&c.merged[(c.merges + uint32_t(s)) & (kRowsL - 1)]);
             }
-            if (s >= 2 && polls) put(s - 2, k0, k1);
+            if (s >= 2) put(s - 2, k0, k1);  // (after a give-up in wait_merged: an earlier row's keys)
         }
         // the last two rows
         tile_sync(t);
