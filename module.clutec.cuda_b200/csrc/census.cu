@@ -139,7 +139,7 @@ struct BmCensusHandle : ct_handle {
     ct_census_match_params par{};
     uint64_t* desc = nullptr;      // [2][H][pitch] census descriptors of left, right
     size_t desc_pitch = 0;         // elements
-    uint32_t* keys = nullptr;      // ceil(D/64) planes of W*H merge keys
+    uint32_t* keys = nullptr;      // ceil(D/64) planes of W*H merge keys, or one plane of right-view keys, of one call
     uint32_t* counters = nullptr;  // one per (strip, column tile); 0 between calls
     uint32_t* rl_keys = nullptr;   // right-view keys of the fused pass, rows of cm::rl_pitch_words(W)
     bool rl_max_keys = false;      // kind of the keys in the plane, and tags used since it was last set (next_tag)
@@ -224,7 +224,7 @@ int next_tag(BmCensusHandle* h, bool max_keys, cudaStream_t s, uint32_t* tag) {
 // Maps from the right-view keys of a pass: the right-view map (disp_rl) and the
 // cross-check of the left map lr (disp_checked), each when given.
 template <typename T, typename Keys>
-int launch_rl_check(BmCensusHandle* h, Keys how, const ct_image* lr, const ct_image* disp_rl,
+int launch_rl_check(BmCensusHandle* h, const uint32_t* keys, Keys how, const ct_image* lr, const ct_image* disp_rl,
                     const ct_image* disp_checked, int tol, cudaStream_t s) {
     using namespace cm;
     const int W = h->fmt.width, H = h->fmt.height;
@@ -240,19 +240,18 @@ int launch_rl_check(BmCensusHandle* h, Keys how, const ct_image* lr, const ct_im
     cfg.numAttrs = 1;
     auto ptr = [](const ct_image* im) { return im ? static_cast<T*>(im->ptr) : nullptr; };
     auto pitch = [](const ct_image* im) { return im ? im->pitch_bytes : size_t(0); };
-    CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, rl_check_kernel<T, Keys>, static_cast<const uint32_t*>(h->rl_keys),
-                                   rl_pitch_words(W), how, W, H, int(kAR), ptr(disp_rl), pitch(disp_rl),
-                                   static_cast<const T*>(ptr(lr)), pitch(lr), ptr(disp_checked),
-                                   pitch(disp_checked), tol));
+    CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, rl_check_kernel<T, Keys>, keys, rl_pitch_words(W), how, W, H, int(kAR),
+                                   ptr(disp_rl), pitch(disp_rl), static_cast<const T*>(ptr(lr)), pitch(lr),
+                                   ptr(disp_checked), pitch(disp_checked), tol));
     CT_LAUNCH_CHECK();
     return CT_OK;
 }
 
 template <typename Keys>
-int rl_check(BmCensusHandle* h, int type, Keys how, const ct_image* lr, const ct_image* disp_rl,
+int rl_check(BmCensusHandle* h, const uint32_t* keys, int type, Keys how, const ct_image* lr, const ct_image* disp_rl,
              const ct_image* disp_checked, int tol, cudaStream_t s) {
-    return type == CT_PIX_U8 ? launch_rl_check<uint8_t>(h, how, lr, disp_rl, disp_checked, tol, s)
-                             : launch_rl_check<uint16_t>(h, how, lr, disp_rl, disp_checked, tol, s);
+    return type == CT_PIX_U8 ? launch_rl_check<uint8_t>(h, keys, how, lr, disp_rl, disp_checked, tol, s)
+                             : launch_rl_check<uint16_t>(h, keys, how, lr, disp_rl, disp_checked, tol, s);
 }
 
 // process_lr in one matching pass: the left-to-right kernel decides both
@@ -264,7 +263,7 @@ int census_process_fused(BmCensusHandle* h, const ct_image* lr, const ct_image* 
     uint32_t tag;
     if (int rc = next_tag(h, false, s, &tag)) return rc;
     if (int rc = census_match_pass_maps(h, 0, lr, h->tm_lb, h->tm_rm, s, nullptr, &tag)) return rc;
-    return rl_check(h, lr->type, cm::MinKeys{tag}, lr, disp_rl, disp_checked, tol, s);
+    return rl_check(h, h->rl_keys, lr->type, cm::MinKeys{tag}, lr, disp_rl, disp_checked, tol, s);
 }
 
 // One pass on the tensor cores over the handle's row-major descriptors: the
@@ -273,14 +272,16 @@ int census_process_fused(BmCensusHandle* h, const ct_image* lr, const ct_image* 
 int census_process_tc(BmCensusHandle* h, const ct_image* lr, const ct_image* disp_rl, const ct_image* disp_checked,
                       int tol, cudaStream_t s) {
     const bool need_r = disp_rl || disp_checked;
+    uint32_t* keys = h->rl_keys;
     uint32_t tag = 0;
     if (need_r && lr) {
         if (int rc = next_tag(h, true, s, &tag)) return rc;
     } else if (need_r) {
-        // the right view alone: a plane set for this call only, so that the
-        // call can be captured and replayed as its CUDA-core pass can
-        CT_CUDA_TRY(cudaMemsetAsync(h->rl_keys, 0, cm::rl_pitch_words(h->fmt.width) * size_t(h->fmt.height) * 4, s));
-        h->rl_tags_used = cm::kRLTags;  // the next call sets it again
+        // the right view alone: a plane set for this call only, in scratch that
+        // no other call reads, so that the call can be captured and replayed
+        // between any others as its CUDA-core pass can
+        keys = h->keys;
+        CT_CUDA_TRY(cudaMemsetAsync(keys, 0, cm::rl_pitch_words(h->fmt.width) * size_t(h->fmt.height) * 4, s));
         tag = 1u << cm::kRLTagShift;
     }
     ctc::Args a{};
@@ -293,7 +294,7 @@ int census_process_tc(BmCensusHandle* h, const ct_image* lr, const ct_image* dis
     if (lr) {
         a.out = lr->ptr; a.out_pitch = lr->pitch_bytes; a.out_type = lr->type;
     }
-    a.r_keys = need_r ? h->rl_keys : nullptr;
+    a.r_keys = need_r ? keys : nullptr;
     a.key_pitch = cm::rl_pitch_words(a.W);
     a.tag = tag;
     a.status = h->d_status;
@@ -311,7 +312,8 @@ int census_process_tc(BmCensusHandle* h, const ct_image* lr, const ct_image* dis
     CT_CUDA_TRY(cudaLaunchKernelEx(&cfg, census_tc_kernel, a));
     CT_LAUNCH_CHECK();
     if (!need_r) return CT_OK;
-    return rl_check(h, (disp_rl ? disp_rl : disp_checked)->type, cm::MaxKeys{tag, a.dmin}, lr, disp_rl, disp_checked, tol, s);
+    return rl_check(h, keys, (disp_rl ? disp_rl : disp_checked)->type, cm::MaxKeys{tag, a.dmin}, lr, disp_rl, disp_checked,
+                    tol, s);
 }
 
 int census_match_pass(BmCensusHandle* h, int dir, const ct_image* disp, cudaStream_t s,
@@ -451,7 +453,8 @@ int ct_bm_census_configure(ct_handle* hh, int32_t device, const ct_format* fmt, 
     h->desc_pitch = cm::planar_pitch(W);  // pair-planar layout
     if (cudaMalloc(&h->desc, 2 * h->desc_pitch * H * 8) != cudaSuccess) return fail(CT_ENOMEM, "descriptor scratch");
     const size_t zplanes = (p->disp_count + (p->disp_min & 1) + cm::kDPC - 1) / cm::kDPC;
-    if (cudaMalloc(&h->keys, zplanes * W * H * 4) != cudaSuccess) return fail(CT_ENOMEM, "key scratch");
+    if (cudaMalloc(&h->keys, std::max(zplanes * W, cm::rl_pitch_words(W)) * H * 4) != cudaSuccess)
+        return fail(CT_ENOMEM, "key scratch");
     // counters for the shortest strips any launch shape uses (11 rows)
     const size_t ngroups = size_t((H + 10) / 11) * ((W + cm::kTWO - 1) / cm::kTWO);
     if (cudaMalloc(&h->counters, ngroups * 4) != cudaSuccess) return fail(CT_ENOMEM, "counter scratch");
