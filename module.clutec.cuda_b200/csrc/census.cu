@@ -266,6 +266,17 @@ int census_process_fused(BmCensusHandle* h, const ct_image* lr, const ct_image* 
     return rl_check(h, h->rl_keys, lr->type, cm::MinKeys{tag}, lr, disp_rl, disp_checked, tol, s);
 }
 
+// Whether `s` is being captured into a graph: its replays repeat a call with the
+// same tag, and unknown to the handle's count of tags.
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();  // the call itself will report what is wrong with the stream
+        return false;
+    }
+    return st == cudaStreamCaptureStatusActive;
+}
+
 // One pass on the tensor cores over the handle's row-major descriptors: the
 // left map (lr), the right-view map and the cross-check of lr, each when given
 // (lr is, with the cross-check).
@@ -274,12 +285,12 @@ int census_process_tc(BmCensusHandle* h, const ct_image* lr, const ct_image* dis
     const bool need_r = disp_rl || disp_checked;
     uint32_t* keys = h->rl_keys;
     uint32_t tag = 0;
-    if (need_r && lr) {
+    if (need_r && lr && !capturing(s)) {
         if (int rc = next_tag(h, true, s, &tag)) return rc;
     } else if (need_r) {
-        // the right view alone: a plane set for this call only, in scratch that
-        // no other call reads, so that the call can be captured and replayed
-        // between any others as its CUDA-core pass can
+        // captured, or the right view alone: a plane set for this call only, in
+        // scratch that no other call reads, so that replays can run between any
+        // other calls
         keys = h->keys;
         CT_CUDA_TRY(cudaMemsetAsync(keys, 0, cm::rl_pitch_words(h->fmt.width) * size_t(h->fmt.height) * 4, s));
         tag = 1u << cm::kRLTagShift;
@@ -580,7 +591,7 @@ int ct_bm_census_process_lr(ct_handle* hh, const ct_image* disp_lr, const ct_ima
     const ct_image* lr = disp_lr ? disp_lr : &tlr;
     if (tc) return census_process_tc(h, need_lr ? lr : nullptr, disp_rl, disp_checked, tol, s);
     const ct_image* rl = disp_rl ? disp_rl : &trl;
-    if (need_lr && need_rl && h->fuse_rl)  // the same maps as two passes
+    if (need_lr && need_rl && h->fuse_rl && !capturing(s))  // the same maps as two passes
         return census_process_fused(h, lr, disp_rl, disp_checked, tol, s);
     {
         if (need_lr)

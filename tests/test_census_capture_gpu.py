@@ -66,3 +66,30 @@ def test_right_view_replays_between_direct_calls(ct, cuda, scenes, cuda_cores):
             g.replay()
             _same(alone, want[1], f"replay {k}")
     assert m.device_status() == 0
+
+
+@pytest.mark.parametrize("cuda_cores", [False, True])
+def test_checked_replays_between_direct_calls(ct, cuda, scenes, cuda_cores):
+    """Every replay's keys are its own: neither an earlier replay's, with the
+    same tag, nor those of the direct calls between."""
+    scenes, left, right = scenes
+    m = ct.BlockMatcherCensus()
+    m.configure(0, W, H, D)
+    if cuda_cores:
+        m.set_tuning(36, 4)
+    out, direct = _maps(ct, cuda), _maps(ct, cuda)
+    m.process_lr(left, right, *out, tol=1)
+    g = _capture(lambda: m.process_lr(left, right, *out, tol=1))
+    for k in range(40):
+        dl, dr, want = scenes[k % 3]
+        left.copy_(dl)
+        right.copy_(dr)
+        g.replay()
+        for o, w, name in zip(out, want, ("left", "right", "checked")):
+            _same(o, w, f"replay {k} {name}")
+        if k % 2:
+            dl, dr, want = scenes[(k + 1) % 3]
+            m.process_lr(dl, dr, *direct, tol=1)
+            for o, w, name in zip(direct, want, ("left", "right", "checked")):
+                _same(o, w, f"call {k} {name}")
+    assert m.device_status() == 0
