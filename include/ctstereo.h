@@ -211,13 +211,19 @@ int ct_bm_census_process_curves(ct_handle* h, const ct_image* disp, const ct_cur
  * `stream`. (No counterpart in the reference, whose launch shapes are
  * compile-time SConfig constants, BlockMatcherNCC.h:43-79.) */
 int ct_bm_census_autotune(ct_handle* h, const ct_image* left, const ct_image* right, ct_stream stream);
-/* The handle's current launch shape of the CUDA-core kernel (strip height in
- * rows, disparities per warp); either pointer may be NULL. (The tensor-core
- * kernel, which runs where it is the faster one, has one shape per size.) */
+/* The handle's current tuning; either pointer may be NULL. *strip_height is the
+ * CUDA-core kernel's strip height in rows (11..511) plus a CT_TUNING_TC_* for
+ * each kind of pass that runs on the tensor cores instead (which have one shape
+ * per size); *disp_per_warp is the CUDA-core kernel's (4 or 8). Both are meant to
+ * be saved and given to ct_bm_census_set_tuning as they are: *strip_height % 5 is
+ * always 1, as of a plain strip height. */
+#define CT_TUNING_TC_LEFT 20480  /* the left view: ct_bm_census_process, and ..._process_lr */
+#define CT_TUNING_TC_RIGHT 40960 /* the right view alone */
 int ct_bm_census_tuning(ct_handle* h, int32_t* strip_height, int32_t* disp_per_warp);
-/* Sets the launch shape (e.g. from a saved tuning table): strip_height with
- * strip_height + 4 a multiple of 5 (11..511), disp_per_warp 4 or 8, and selects
- * the CUDA-core kernel. Results do not depend on it. */
+/* Sets the tuning (e.g. from a saved table): values of ct_bm_census_tuning, or a
+ * launch shape of the CUDA-core kernel, which then runs every pass: strip_height
+ * with strip_height + 4 a multiple of 5 (11..511), disp_per_warp 4 or 8. Results
+ * do not depend on it. */
 int ct_bm_census_set_tuning(ct_handle* h, int32_t strip_height, int32_t disp_per_warp);
 /* ct_bm_census_process_lr computes both directions in one matching pass by
  * default: the 5x5 Hamming cost of right pixel x_R at disparity e is the

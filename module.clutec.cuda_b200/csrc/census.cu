@@ -670,7 +670,8 @@ int ct_bm_census_tuning(ct_handle* hh, int32_t* strip_height, int32_t* disp_per_
     auto* h = as<BmCensusHandle>(hh, Kind::BmCensus);
     if (!h) return fail(CT_ESTATE, "not a census matcher handle");
     if (!h->configured) return fail(CT_ESTATE, "tuning before configure");
-    if (strip_height) *strip_height = h->th;
+    if (strip_height)
+        *strip_height = h->th + (h->use_tc ? CT_TUNING_TC_LEFT : 0) + (h->use_tc_right ? CT_TUNING_TC_RIGHT : 0);
     if (disp_per_warp) *disp_per_warp = h->dpw;
     return CT_OK;
 }
@@ -688,12 +689,16 @@ int ct_bm_census_set_tuning(ct_handle* hh, int32_t strip_height, int32_t disp_pe
     clear_error();
     auto* h = as<BmCensusHandle>(hh, Kind::BmCensus);
     if (!h) return fail(CT_ESTATE, "not a census matcher handle");
-    if (strip_height < 11 || strip_height > 511 || (strip_height + 2 * cm::kAR) % cm::kRB != 0)
-        return fail(CT_EINVAL, "strip_height must be 11..511 with strip_height + 4 a multiple of 5");
+    // (the kernels' values are multiples of 5 << 12, above any strip height)
+    const int th = strip_height % CT_TUNING_TC_LEFT, tc = strip_height / CT_TUNING_TC_LEFT;
+    if (strip_height < 11 || tc > 3 || th < 11 || th > 511 || (th + 2 * cm::kAR) % cm::kRB != 0)
+        return fail(CT_EINVAL, "strip_height must be 11..511 with strip_height + 4 a multiple of 5, "
+                               "or a value of ct_bm_census_tuning");
     if (disp_per_warp != 4 && disp_per_warp != 8) return fail(CT_EINVAL, "disp_per_warp must be 4 or 8");
-    h->th = strip_height;
+    h->th = th;
     h->dpw = disp_per_warp;
-    h->use_tc = h->use_tc_right = false;  // the shape asked for is the CUDA-core kernel's
+    h->use_tc = tc & 1;
+    h->use_tc_right = tc & 2;
     return CT_OK;
 }
 

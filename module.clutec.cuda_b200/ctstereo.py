@@ -118,6 +118,7 @@ class ct_color_params(C.Structure):
 
 
 CT_CONFNET_PARAMS = 12673
+CT_TUNING_TC_LEFT, CT_TUNING_TC_RIGHT = 20480, 40960
 
 
 class ct_pipe_rates(C.Structure):
@@ -371,6 +372,7 @@ class BlockMatcherCensus(_Driver):
         return self.tuning()
 
     def set_tuning(self, strip_height: int, disp_per_warp: int):
+        """A saved tuning(), or a launch shape of the CUDA-core kernel, which then runs every pass."""
         check(lib().ct_bm_census_set_tuning(self._h, strip_height, disp_per_warp))
 
     def set_fused_lr(self, enable: bool):
@@ -378,6 +380,8 @@ class BlockMatcherCensus(_Driver):
         check(lib().ct_bm_census_set_fused_lr(self._h, 1 if enable else 0))
 
     def tuning(self):
+        """For set_tuning on another handle: launch shape of the CUDA-core kernel and, added to the
+        strip height, CT_TUNING_TC_* for the passes that run on the tensor cores."""
         th, dpw = C.c_int32(), C.c_int32()
         check(lib().ct_bm_census_tuning(self._h, C.byref(th), C.byref(dpw)))
         return {"strip_height": th.value, "disp_per_warp": dpw.value}
