@@ -206,9 +206,9 @@ int ct_bm_census_process_curves(ct_handle* h, const ct_image* disp, const ct_cur
 
 /* Autotuner: times the CUDA-core kernel's variants (4 or 8 disparities per
  * warp) and strip heights, and the tensor-core kernel, for this handle's (W, H,
- * D, direction) on the given images, keeps the fastest in the handle for later
- * process calls. Synchronises
- * `stream`. (No counterpart in the reference, whose launch shapes are
+ * D, direction) on the given images, and the pass of both directions
+ * (ct_bm_census_process_lr) on either kernel, and keeps the fastest of each in
+ * the handle for later calls. Synchronises `stream`. (No counterpart in the reference, whose launch shapes are
  * compile-time SConfig constants, BlockMatcherNCC.h:43-79.) */
 int ct_bm_census_autotune(ct_handle* h, const ct_image* left, const ct_image* right, ct_stream stream);
 /* The handle's current tuning; either pointer may be NULL. *strip_height is the
@@ -217,8 +217,9 @@ int ct_bm_census_autotune(ct_handle* h, const ct_image* left, const ct_image* ri
  * per size); *disp_per_warp is the CUDA-core kernel's (4 or 8). Both are meant to
  * be saved and given to ct_bm_census_set_tuning as they are: *strip_height % 5 is
  * always 1, as of a plain strip height. */
-#define CT_TUNING_TC_LEFT 20480  /* the left view: ct_bm_census_process, and ..._process_lr */
+#define CT_TUNING_TC_LEFT 20480  /* the left view alone */
 #define CT_TUNING_TC_RIGHT 40960 /* the right view alone */
+#define CT_TUNING_TC_LR 81920    /* both: ct_bm_census_process_lr in one pass */
 int ct_bm_census_tuning(ct_handle* h, int32_t* strip_height, int32_t* disp_per_warp);
 /* Sets the tuning (e.g. from a saved table): values of ct_bm_census_tuning, or a
  * launch shape of the CUDA-core kernel, which then runs every pass: strip_height

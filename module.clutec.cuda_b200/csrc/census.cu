@@ -153,8 +153,9 @@ struct BmCensusHandle : ct_handle {
     int dpw = 4;   // disparities per warp (kernel variant)
     ctc::Shape tc{};   // tile shape and strip height of the tensor-core pass
     int tc_rows = 0;
-    bool use_tc = false;        // left-to-right (and fused) passes on the tensor cores (tc_faster)
-    bool use_tc_right = false;  // and passes for the right view alone
+    // passes on the tensor cores (tc_faster): for the left view alone, for the
+    // right view alone, for both
+    bool use_tc = false, use_tc_right = false, use_tc_lr = false;
     uint64_t* left_desc() const { return desc; }
     uint64_t* right_desc() const { return desc + (size_t)fmt.height * desc_pitch; }
 };
@@ -478,7 +479,7 @@ int ct_bm_census_configure(ct_handle* hh, int32_t device, const ct_format* fmt, 
     CT_CUDA_TRY(cudaMemset(h->rl_keys, 0xFF, rl_bytes));
     h->rl_max_keys = false;
     h->rl_tags_used = 0;
-    h->use_tc = tc_faster(W, H, p->disp_count, true);
+    h->use_tc = h->use_tc_lr = tc_faster(W, H, p->disp_count, true);
     h->use_tc_right = tc_faster(W, H, p->disp_count, false);
     h->tc = ctc::pick_shape(W, p->disp_count);
     h->tc_rows = ctc::pick_rows(H, h->tc.tiles_x, sm_count(device));
@@ -582,7 +583,7 @@ int ct_bm_census_process_lr(ct_handle* hh, const ct_image* disp_lr, const ct_ima
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     h->last_stream = s;
     const bool need_lr = disp_lr || disp_checked, need_rl = disp_rl || disp_checked;
-    const bool tc = need_lr ? h->use_tc && (!need_rl || h->fuse_rl) : h->use_tc_right;
+    const bool tc = !need_lr ? h->use_tc_right : need_rl ? h->use_tc_lr && h->fuse_rl : h->use_tc;
     if (int rc = census_both(h, left, right, s, tc ? 0 : 1)) return rc;
     const int W = h->fmt.width, H = h->fmt.height;
     ct_image tlr{h->tmp_lr, h->tmp_pitch, W, H, t, 0};
@@ -651,17 +652,23 @@ int ct_bm_census_autotune(ct_handle* hh, const ct_image* left, const ct_image* r
         }
         if (rc) break;
     }
-    // the tensor-core pass, on row-major descriptors
-    if (!rc && !(rc = census_both(h, left, right, s, 0))) {
-        float t;
-        rc = timed([&] { return dir == 0 ? census_process_tc(h, &out, nullptr, nullptr, 0, s)
-                                         : census_process_tc(h, nullptr, &out, nullptr, 0, s); }, &t);
-        if (!rc) (dir == 0 ? h->use_tc : h->use_tc_right) = t < best_ms;
+    h->th = best_th;
+    h->dpw = best_dpw;
+    // both views' maps in one pass, then the tensor-core passes, on row-major
+    // descriptors
+    ct_image out_rl{h->tmp_rl, h->tmp_pitch, W, H, CT_PIX_U16, 0};
+    float lr_ms, t, t_lr;
+    if (!rc) rc = timed([&] { return census_process_fused(h, &out, &out_rl, nullptr, 0, s); }, &lr_ms);
+    if (!rc) rc = census_both(h, left, right, s, 0);
+    if (!rc) rc = timed([&] { return dir == 0 ? census_process_tc(h, &out, nullptr, nullptr, 0, s)
+                                              : census_process_tc(h, nullptr, &out, nullptr, 0, s); }, &t);
+    if (!rc) rc = timed([&] { return census_process_tc(h, &out, &out_rl, nullptr, 0, s); }, &t_lr);
+    if (!rc) {
+        (dir == 0 ? h->use_tc : h->use_tc_right) = t < best_ms;
+        h->use_tc_lr = t_lr < lr_ms;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    h->th = best_th;
-    h->dpw = best_dpw;
     return rc;
 }
 
@@ -671,7 +678,8 @@ int ct_bm_census_tuning(ct_handle* hh, int32_t* strip_height, int32_t* disp_per_
     if (!h) return fail(CT_ESTATE, "not a census matcher handle");
     if (!h->configured) return fail(CT_ESTATE, "tuning before configure");
     if (strip_height)
-        *strip_height = h->th + (h->use_tc ? CT_TUNING_TC_LEFT : 0) + (h->use_tc_right ? CT_TUNING_TC_RIGHT : 0);
+        *strip_height = h->th + (h->use_tc ? CT_TUNING_TC_LEFT : 0) + (h->use_tc_right ? CT_TUNING_TC_RIGHT : 0) +
+                        (h->use_tc_lr ? CT_TUNING_TC_LR : 0);
     if (disp_per_warp) *disp_per_warp = h->dpw;
     return CT_OK;
 }
@@ -691,7 +699,7 @@ int ct_bm_census_set_tuning(ct_handle* hh, int32_t strip_height, int32_t disp_pe
     if (!h) return fail(CT_ESTATE, "not a census matcher handle");
     // (the kernels' values are multiples of 5 << 12, above any strip height)
     const int th = strip_height % CT_TUNING_TC_LEFT, tc = strip_height / CT_TUNING_TC_LEFT;
-    if (strip_height < 11 || tc > 3 || th < 11 || th > 511 || (th + 2 * cm::kAR) % cm::kRB != 0)
+    if (strip_height < 11 || tc > 7 || th < 11 || th > 511 || (th + 2 * cm::kAR) % cm::kRB != 0)
         return fail(CT_EINVAL, "strip_height must be 11..511 with strip_height + 4 a multiple of 5, "
                                "or a value of ct_bm_census_tuning");
     if (disp_per_warp != 4 && disp_per_warp != 8) return fail(CT_EINVAL, "disp_per_warp must be 4 or 8");
@@ -699,6 +707,7 @@ int ct_bm_census_set_tuning(ct_handle* hh, int32_t strip_height, int32_t disp_pe
     h->dpw = disp_per_warp;
     h->use_tc = tc & 1;
     h->use_tc_right = tc & 2;
+    h->use_tc_lr = tc & 4;
     return CT_OK;
 }
 

@@ -118,7 +118,7 @@ class ct_color_params(C.Structure):
 
 
 CT_CONFNET_PARAMS = 12673
-CT_TUNING_TC_LEFT, CT_TUNING_TC_RIGHT = 20480, 40960
+CT_TUNING_TC_LEFT, CT_TUNING_TC_RIGHT, CT_TUNING_TC_LR = 20480, 40960, 81920
 
 
 class ct_pipe_rates(C.Structure):

@@ -50,6 +50,29 @@ def test_saved_tuning_runs_the_same_kernels(ct, oracle, cuda, W, H, D, tune):
     assert a.device_status() == 0 and b.device_status() == 0
 
 
+def test_each_kind_of_pass_has_a_kernel_of_its_own(ct, oracle, cuda):
+    """(The autotuner times the pass of both views by itself: which kernel is the
+    faster one for the left view alone does not decide it.)"""
+    W, H, D = 333, 47, 100
+    L, R, _, _ = ct.synth_pair(2, 5, W, H, D - 1)
+    dl, dr = to_dev(L, cuda), to_dev(R, cuda)
+    lr, rl = (oracle.to_u16(oracle.match_census(L, R, D, 2, left)[0]) for left in (True, False))
+    want = lr, rl, oracle.crosscheck_codes(lr, rl, 1, True, frame=False)[0]
+    m = ct.BlockMatcherCensus()
+    m.configure(0, W, H, D)
+    out = [ct.alloc_image(H, W, torch.int16, cuda) for _ in range(3)]
+    for k in range(8):
+        m.set_tuning(36 + k * ct.CT_TUNING_TC_LEFT, 4)
+        assert _on_tensor_cores(ct, cuda, m, dl, dr) == {"left": bool(k & 1), "right": bool(k & 2),
+                                                         "checked": bool(k & 4)}
+        m.process_lr(dl, dr, disp_lr=out[0])
+        m.process_lr(dl, dr, disp_rl=out[1])
+        m.process_lr(dl, dr, disp_checked=out[2])
+        for o, w in zip(out, want):
+            np.testing.assert_array_equal(o.cpu().numpy().view(np.uint16), w)
+    assert m.device_status() == 0
+
+
 def test_tunings_of_no_kernel_are_refused(ct, cuda):
     m = ct.BlockMatcherCensus()
     m.configure(0, 160, 96, 64)
