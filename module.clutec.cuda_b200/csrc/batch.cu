@@ -153,7 +153,6 @@ __global__ void __launch_bounds__(kCheckT) check_batch_kernel(const PairDev* pai
 
 __global__ void __launch_bounds__(ctc::kNT, 1)
     match_batch_kernel(const PairDev* pairs, int n, int total_items, unsigned* queue, uint32_t polls, int32_t* status) {
-    constexpr int NT = ctc::kNT;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ int s_item;
     ctc::Cta c(smem_raw);

@@ -176,26 +176,16 @@ __device__ __forceinline__ void store_disp(void* out, size_t pitch, int type, in
 }
 
 // A CTA's piece of work: column tile bx of nbx, strip by, disparity block bz
-// of nbz. The single-image kernel takes it from blockIdx / gridDim; the
-// batched persistent kernel from its work queue.
+// of nbz.
 struct Tile {
     int bx, by, bz, nbx, nbz;
 };
 
-// Result of one tile: whether this CTA wrote final disparities for its
-// (strip, column tile) group (always when nbz == 1; the last arriver
-// otherwise), and whether a tile load timed out.
-struct TileResult {
-    bool group_done;
-    bool aborted;
-};
-
 template <int DIR, bool EDGE, int DPW, bool CURVE, bool RL = false>
-__device__ __forceinline__ TileResult match_body(const CUtensorMap* tmB, const CUtensorMap* tmM,
-                                                 const MatchArgs& a, const Tile& t, uint64_t* sB, uint64_t* sM,
-                                                 uint32_t* sKey, uint64_t* bars, int* sflag, const uint32_t* par,
-                                                 int nb, int rows_here, int xs, int y0, int ye0, int dz0, int ms,
-                                                 uint32_t* sKeyRL = nullptr) {
+__device__ __forceinline__ void match_body(const CUtensorMap* tmB, const CUtensorMap* tmM, const MatchArgs& a,
+                                           const Tile& t, uint64_t* sB, uint64_t* sM, uint32_t* sKey, uint64_t* bars,
+                                           int* sflag, int nb, int rows_here, int xs, int y0, int ye0, int dz0, int ms,
+                                           uint32_t* sKeyRL = nullptr) {
     static_assert(!RL || (DIR == 0 && !CURVE), "the fused right-to-left keys ride on the plain left-to-right pass");
     static_assert(!RL || DPW % 4 == 0, "the right-view key interleave assumes warps of 4k disparities");
     using VT = Var<DPW>;
@@ -481,11 +471,11 @@ __device__ __forceinline__ TileResult match_body(const CUtensorMap* tmB, const C
 
     // Cost row i = kBR * b + r. Before row i is added, V holds rows i-5..i-1:
     // the window of output row i - 5, whose keys go to buffer b & 1, slot r.
-    // Stage s is used by batches s, s + 2, ...: its (b >> 1)-th use in this
-    // tile completes phase par[s] + (b >> 1) of its mbarrier.
+    // Stage s is used by batches s, s + 2, ...: its (b >> 1)-th use completes
+    // phase b >> 1 of its mbarrier.
     for (int b = 0; b < nb; ++b) {
         const int s = b & 1;
-        if (!dev::mbar_wait_bounded(&bars[s], (par[s] + (b >> 1)) & 1)) *sflag = 1;
+        if (!dev::mbar_wait_bounded(&bars[s], (b >> 1) & 1)) *sflag = 1;
         if (warp_active) {
             if (b == 0) {
 #pragma unroll
@@ -505,12 +495,12 @@ __device__ __forceinline__ TileResult match_body(const CUtensorMap* tmB, const C
         if (*sflag) {     // a tile load never arrived: report and leave together
             if (tid == 0) {
                 dev::report(a.status, CT_ETIMEOUT);
-                if (b + 1 < nb) dev::mbar_wait_bounded(&bars[s ^ 1], (par[s ^ 1] + ((b + 1) >> 1)) & 1);
+                if (b + 1 < nb) dev::mbar_wait_bounded(&bars[s ^ 1], ((b + 1) >> 1) & 1);
                 if (t.nbz > 1 && a.merge_last) {  // keep the group counter consistent
                     if (atomicAdd(group_counter, 1u) == unsigned(t.nbz) - 1) *group_counter = 0u;
                 }
             }
-            return TileResult{false, true};
+            return;
         }
         if (tid == 0 && b + 2 < nb) {
             dev::fence_proxy_async();
@@ -527,8 +517,7 @@ __device__ __forceinline__ TileResult match_body(const CUtensorMap* tmB, const C
     flush(nb & 1, kBR * nb - kRB, 0, 1);
     flush_rl(nb & 1, kBR * nb - kRB, 0, 1);
 
-    if (t.nbz == 1) return TileResult{true, false};
-    if (!a.merge_last) return TileResult{false, false};
+    if (t.nbz == 1 || !a.merge_last) return;
     // The last CTA of this (strip, column tile) group merges the groups' key
     // planes. Writers fence before counting; the merger fences after.
     __syncthreads();
@@ -553,10 +542,9 @@ __device__ __forceinline__ TileResult match_body(const CUtensorMap* tmB, const C
             store_disp(a.out, a.out_pitch, a.out_type, x, y, valid, best, a.dmin);
         }
     }
-    return TileResult{last, false};
 }
 
-// Shared-memory carve-up common to the single-image and the batched kernels.
+// Shared-memory carve-up.
 struct Smem {
     uint64_t* sB;     // [2 stages][kBR][2][kPB][2]
     uint64_t* sM;     // [2 stages][kBR][2][kPM][2]
@@ -573,11 +561,10 @@ struct Smem {
           sKeyRL(reinterpret_cast<uint32_t*>(raw + rl_offset())) {}
 };
 
-// Runs one tile. The mbarriers must be initialised; par[s] counts the phases
-// stage s has completed so far in this CTA and is advanced here.
+// Runs the CTA's tile. The mbarriers must be initialised.
 template <int DIR, int DPW, bool CURVE = false, bool RL = false>
-__device__ TileResult run_tile(const CUtensorMap* tmB, const CUtensorMap* tmM, const MatchArgs& a, const Tile& t,
-                               const Smem& sm, uint32_t* par) {
+__device__ void run_tile(const CUtensorMap* tmB, const CUtensorMap* tmM, const MatchArgs& a, const Tile& t,
+                         const Smem& sm) {
     const int tid = threadIdx.x;
     const int xs = t.bx * kTWO - kAR;             // first V column
     const int y0 = t.by * a.th;                   // first output row
@@ -608,15 +595,12 @@ __device__ TileResult run_tile(const CUtensorMap* tmB, const CUtensorMap* tmM, c
             dev::tma_load_4d(sm.sM + b * (kStageM / 8), tmM, 0, (ms >> 1) >> 1, 0, ye0 + b * kBR, &sm.bars[b]);
         }
     }
-    const TileResult res =
-        interior ? match_body<DIR, false, DPW, CURVE, RL>(tmB, tmM, a, t, sm.sB, sm.sM, sm.sKey, sm.bars, sm.sflag,
-                                                          par, nb, rows_here, xs, y0, ye0, dz0, ms, sm.sKeyRL)
-                 : match_body<DIR, true, DPW, CURVE, RL>(tmB, tmM, a, t, sm.sB, sm.sM, sm.sKey, sm.bars, sm.sflag,
-                                                         par, nb, rows_here, xs, y0, ye0, dz0, ms, sm.sKeyRL);
-    par[0] += (nb + 1) / 2;
-    par[1] += nb / 2;
-    __syncthreads();  // the next tile reuses the shared memory
-    return res;
+    if (interior)
+        match_body<DIR, false, DPW, CURVE, RL>(tmB, tmM, a, t, sm.sB, sm.sM, sm.sKey, sm.bars, sm.sflag, nb, rows_here,
+                                               xs, y0, ye0, dz0, ms, sm.sKeyRL);
+    else
+        match_body<DIR, true, DPW, CURVE, RL>(tmB, tmM, a, t, sm.sB, sm.sM, sm.sKey, sm.bars, sm.sflag, nb, rows_here,
+                                              xs, y0, ye0, dz0, ms, sm.sKeyRL);
 }
 
 __device__ __forceinline__ void init_barriers(const Smem& sm) {
@@ -644,9 +628,8 @@ __global__ void __launch_bounds__(Var<DPW>::kNT, 1)
     // This launch is itself programmatic: the previous kernel (census or the
     // other direction) must be complete before any global read or write.
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    uint32_t par[2] = {0, 0};
     const Tile t{int(blockIdx.x), int(blockIdx.y), int(blockIdx.z), int(gridDim.x), int(gridDim.z)};
-    run_tile<DIR, DPW, CURVE, RL>(&tmB, &tmM, a, t, sm, par);
+    run_tile<DIR, DPW, CURVE, RL>(&tmB, &tmM, a, t, sm);
 }
 
 // Map code of a disparity, or of none.
