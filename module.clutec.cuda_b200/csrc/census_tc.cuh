@@ -188,21 +188,21 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
 }
 // Waits for phase `parity` of `bar`, suspended for up to 20 us a poll (waiting
 // warps that poll more often take the maxima's issue slots), for `polls` polls.
-// Returns the polls for the warp's next wait: the same (about a second), or 0
-// once a wait gave up; the warp's lanes agree, and meet, in the vote.
+// Returns the polls for the next wait: the same (about a second), or 0 once a
+// wait gave up.
 constexpr uint32_t kPolls = 1u << 16;
 __device__ __forceinline__ uint32_t wait(uint64_t* bar, uint32_t parity, uint32_t polls) {
     const uint32_t addr = dev::smem_u32(bar);
-    uint32_t done = 0;
     for (uint32_t i = 0; i < polls; ++i) {
+        uint32_t done;
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done)
             : "r"(addr), "r"(parity), "r"(20000u)
             : "memory");
-        if (done) break;
+        if (done) return polls;
     }
-    return __all_sync(0xffffffffu, done) ? polls : 0;
+    return 0;
 }
 __device__ __forceinline__ void arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dev::smem_u32(bar)) : "memory");
@@ -270,9 +270,13 @@ __device__ __forceinline__ float halve(float lo, float hi, bool upper, int mask)
 // are complete, which the MMA warp issued after it joined row k - 3.
 // A warp whose wait gave up (about a second without an answer) keeps taking part
 // in every hand-over, so that the MMA warp, which waits on nothing else, comes
-// to its end and the CTA can report: it reads, stages and writes nothing more,
-// and arrives for a row once the MMA warp has passed the hand-over that the wait
-// stood behind (Cta::passed).
+// to its end and the CTA can report. It arrives for a row once the MMA warp has
+// passed the hand-over that the wait stood behind (Cta::passed), and stages
+// nothing more: every row then leaves a window as it came in, also in MMAs that
+// it did not wait for, so that accumulators read unfinished lie between those of
+// finished rows. Their keys are wrong but as bounded as others: columns outside
+// the band stay below 0 and bid for nothing. (Holding back the keys as well cost
+// 1.6% of a batch.)
 constexpr int kRowBars = 8;
 static_assert(kRowBars >= kSlots && 5 + kRowBars <= 16, "staged rows come round to a barrier after the MMA warp has joined it");
 template <int ID, int N>
@@ -318,11 +322,12 @@ struct Cta {
     // Row s of the tile: its barrier, and the wait for it (nobody waits more
     // than 2 rows behind the MMAs, so 4 barriers leave the phase unambiguous).
     __device__ uint64_t* ready_bar(int t, int s) const { return &ready[4 * t + (step(t, s) & 3)]; }
-    // After it, the MMA warp has passed the hand-overs before the row's MMAs,
-    // also when the wait gave up.
+    // After it, by the whole warp, the MMA warp has passed the hand-overs before
+    // the row's MMAs, also when the wait gave up.
     __device__ uint32_t wait_ready(int t, int s, uint32_t polls) const {
         polls = wait(ready_bar(t, s), (step(t, s) >> 2) & 1, polls);
         if (polls == 0) passed(t, s);
+        __syncwarp();
         return polls;
     }
     __device__ void begin(int t, int s) const { *static_cast<volatile uint32_t*>(misc + 1 + t) = step(t, s) + 1; }
@@ -331,7 +336,6 @@ struct Cta {
     __device__ void passed(int t, int s) const {
         const volatile uint32_t* begun = misc + 1 + t;
         for (uint32_t i = 0; i < (1u << 20) && int32_t(*begun - step(t, s)) <= 0; ++i) __nanosleep(20000);
-        __syncwarp();
     }
 };
 
@@ -463,13 +467,10 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
         auto stage = [&](int k, const uint64_t (&v)[kRowPx]) {
             // row k - 8 left both windows with the last tile's step k - 7
             if (k >= kSlots) polls = c.wait_ready(tiles - 1, k - kSlots + 1, polls);
-            if (polls == 0) {  // (MMAs may still read the slot)
-                row_arrive(k);
-                return;
-            }
             unsigned char* s = c.smem + (k % kSlots) * kSlotBytes;
 #pragma unroll
             for (int j = 0; j < kRowPx; ++j) {
+                if (polls == 0) break;
                 // bit -> sign of a nibble holding 1.0; the order of the bits is
                 // the same for both operands
                 auto e2m1 = [](uint32_t w, int q) { return ((w << q) & 0x88888888u) | 0x22222222u; };
@@ -542,7 +543,8 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
         // to tile 1's warps.
         const int lt = tt - kM, rt = 2 * tt;
         const bool put_l = a.out && lt >= 0 && lt < a.mo && (!share || t == 1) && xl + lt < a.W;
-        const bool put_r = a.r_keys && rt < a.n;  // (n is even)
+        // (n is even; the image's first and last columns have no disparity)
+        const bool put_r = a.r_keys && rt < a.n && xr0 + rt >= 0 && xr0 + rt + 1 < a.W;
         const bool u8 = a.out_type == CT_PIX_U8;
         char* out = static_cast<char*>(a.out) + size_t(y0) * a.out_pitch + (xl + lt) * (u8 ? 1 : 2);
         uint32_t* bids = a.r_keys + size_t(y0) * a.key_pitch + (xr0 + rt);
@@ -588,11 +590,6 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
         float* const put_kr = keyR + q * kKeyN;
         for (int s = 0; s < rows; ++s) {
             polls = c.wait_ready(t, s, polls);
-            if (polls == 0) {  // hand-overs only
-                read_arrive(t);
-                if (share && t == 0 && lane == 0) arrive(&c.merged[(c.merges + uint32_t(s)) & (kRowsL - 1)]);
-                continue;
-            }
             fence_after();
             float rm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             // Maxima of a piece: along the rows into rm, along the columns
@@ -683,20 +680,20 @@ __device__ __forceinline__ bool run_tile(Cta& c, const Args& a, int bx, int by) 
             }
             if (a.out) {
                 const float r0 = halve(rm[0], rm[1], f0, 1), r1 = halve(rm[2], rm[3], f0, 1);
-                put_kl[(s & (kRowsL - 1)) * (4 * kM)] = halve(r0, r1, f1, 2);
+                const float r = halve(r0, r1, f1, 2);
+                put_kl[(s & (kRowsL - 1)) * (4 * kM)] = r;
             }
             if (share && t == 0) {
                 __syncwarp();
                 if (lane == 0) arrive(&c.merged[(c.merges + uint32_t(s)) & (kRowsL - 1)]);
             }
-            if (s >= 2) put(s - 2, k0, k1);  // (after a give-up in wait_merged: an earlier row's keys)
+            if (s >= 2) put(s - 2, k0, k1);
         }
         // the last two rows
         tile_sync(t);
         for (int r = max(rows - 2, 0); r < rows; ++r) {
             float k0 = 0.0f, k1 = 0.0f;
             wait_merged(r);
-            if (polls == 0) break;
             take(r, k0, k1);
             put(r, k0, k1);
         }
