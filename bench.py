@@ -19,10 +19,11 @@ counts pixel x disparity evaluations: 2 directions x W x H x D per step.
   roofline    the dominant kernel (the fused matching pass: each 5x5 Hamming
               cost evaluated once, both directions' winners) timed with CUDA
               events on its stream, against the nominal dense FP4 tensor rate
-              (the window sums are FP4 MMAs: 1280 operations per cost); also
-              the one-direction kernel of process() alone, and both as
-              multiples of the POPC-pipe bound (2 POPC per cost) measured live
-              by ct_probe_pipe_rates, which the CUDA-core kernel had.
+              (the window sums are FP4 MMAs: 1280 operations per cost), or,
+              should the handle's autotuner have preferred the CUDA-core
+              kernel, against the POPC-pipe bound (2 POPC per cost) measured
+              live by ct_probe_pipe_rates; also the one-direction kernel of
+              process() alone, and both as multiples of the POPC bound.
   cpu_baseline  the CPU restatement (OpenMP, all host threads) on the same
               pair, rank 0 only.
 
@@ -66,12 +67,13 @@ def parse():
                     help="held-out 1080p pairs for the confidence-net AUC (default 4 in the census line, 24 in confnet1080)")
     ap.add_argument("--profile", default=None,
                     choices=["census_match", "census_fused", "confnet_infer", "pipelines", "sad640", "ncc1080",
-                             "ncc1080_cuda_cores", "aw1440", "batch64", "compat_ncc1080"],
+                             "ncc1080_cuda_cores", "ncc1080g", "aw1440", "batch64", "compat_ncc1080", "net_gradient"],
                     help="for ncu captures, then exit: census_match or confnet_infer = that kernel twice on the "
                          "1080p D=128 pair; pipelines = the plain L-R pipeline 3x (one fused pass), 3x in two "
-                         "passes, then the learned one 3x; a "
+                         "passes, then the learned one 3x, all on the CUDA-core matcher; a "
                          "configuration name = its step twice (no autotuning, no CPU work); ncc1080_cuda_cores = "
-                         "the ncc1080 step with the window sums on the CUDA cores")
+                         "the ncc1080 step with the window sums on the CUDA cores; net_gradient = the confidence "
+                         "net's gradient of 8192 samples")
     ap.add_argument("--no-configs", action="store_true",
                     help="default run: measure the headline only, without the other configurations")
     return ap.parse_args()
@@ -246,13 +248,14 @@ class ClockSampler:
                 "reasons": reasons, "samples": len(rows)}
 
 
-def traffic_from_profile():
-    """DRAM bytes per launch of the fused census_match_kernel (the headline's
-    dominant kernel) from the committed ncu summary."""
+def traffic_from_profile(tensor_cores):
+    """DRAM bytes per launch of the headline's matching pass (on the tensor or
+    the CUDA cores) from the committed ncu summary."""
     p = ROOT / "profiles" / "census_match_1080p_d128.json"
     if p.exists():
         try:
-            return json.loads(p.read_text()).get("dram_bytes_per_launch")
+            j = json.loads(p.read_text())
+            return (j if tensor_cores else j["cuda_core_fused"]).get("dram_bytes_per_launch")
         except Exception:
             return None
     return None
@@ -535,12 +538,30 @@ def run_ours(args):
     achieved_popc = 2.0 * units_launch / (fused_ms * 1e-3)
     single_popc = 2.0 * units_launch / (match_ms * 1e-3)           # one direction alone, 2 POPC per unit
     launches = 3  # census of both views, the fused matching pass, the right-view map + cross-check
+    tc = ct.tuning_on_tensor_cores(tuning)
+    fp4 = FP4_OPS_PER_COST * units_launch / (fused_ms * 1e-3) / 1e12
+    if tc["both"]:
+        roof = {"bound": "tensor_fp4", "achieved": round(fp4, 2), "peak": FP4_PEAK_TFLOPS, "unit": "TFLOP/s",
+                "frac": round(fp4 / FP4_PEAK_TFLOPS, 4),
+                "kernel": "census_tc_kernel (the matching pass: 5x5 Hamming costs of 1920x1080x128 as FP4 "
+                          "MMAs, left-to-right and right-to-left winners from one accumulator; timed as "
+                          "process_lr(lr, rl) minus the census transform of both views)",
+                "algorithmic_per_unit": "per cost C(x, d) an entering and a leaving window row of 5 x 64 "
+                                        "multiply-adds = 1280 operations, one cost per pixel x disparity for "
+                                        "both directions"}
+    else:
+        roof = {"bound": "popc", "achieved": round(achieved_popc / 1e12, 4), "peak": round(popc_peak / 1e12, 4),
+                "unit": "Tpopc/s", "frac": round(achieved_popc / popc_peak, 4),
+                "kernel": "census_match_kernel (the fused pass on the CUDA cores, both directions' winners; timed as "
+                          "process_lr(lr, rl) minus the census transform of both views)",
+                "algorithmic_per_unit": "2 POPC per cost C(x, d), one cost per pixel x disparity for both directions"}
 
     out = {
         "metric": METRIC, "value": round(value, 1), "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(ms, 4), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "u8 pixels / u64 census / int costs", "data": "synthetic (seeded generator)",
         "config": census_config(), "parallelism": f"replicas x{world}", "launch_shape": tuning,
+        "on_tensor_cores": ct.tuning_on_tensor_cores(tuning),
         "e2e": {"value": round(e2e_stream, 1), "unit": UNIT, "ms_per_step": round(stream_ms, 4),
                 "h2d_bytes_per_step": 2 * W_ * H_, "d2h_bytes_per_step": W_ * H_,
                 "api": "ct_census_stream_submit per frame (pinned host images in, checked map out), "
@@ -550,19 +571,11 @@ def run_ours(args):
                 "serial": {"value": round(e2e, 1), "ms_per_step": round(e2e_ms, 4),
                            "api": "ct_bm_census_process_lr with the copies in line on one stream, "
                                   "L2 flushed before every step"}},
-        "roofline": {"bound": "tensor_fp4", "achieved": round(FP4_OPS_PER_COST * units_launch / (fused_ms * 1e-3) / 1e12, 2),
-                     "peak": FP4_PEAK_TFLOPS, "unit": "TFLOP/s",
-                     "frac": round(FP4_OPS_PER_COST * units_launch / (fused_ms * 1e-3) / 1e12 / FP4_PEAK_TFLOPS, 4),
-                     "traffic": traffic_from_profile(),
-                     "kernel": "census_tc_kernel (the matching pass: 5x5 Hamming costs of 1920x1080x128 as FP4 "
-                               "MMAs, left-to-right and right-to-left winners from one accumulator; timed as "
-                               "process_lr(lr, rl) minus the census transform of both views)",
+        "roofline": {**roof, "traffic": traffic_from_profile(tc["both"]),
                      "kernel_ms": round(fused_ms, 4), "census_transform_ms": round(census_ms, 4),
-                     "algorithmic_per_unit": "per cost C(x, d) an entering and a leaving window row of 5 x 64 "
-                                             "multiply-adds = 1280 operations, one cost per pixel x disparity for "
-                                             "both directions",
                      "popc_equivalent_frac": round(achieved_popc / popc_peak, 4),
-                     "single_direction": {"kernel": "census_tc_kernel (left-to-right alone, process())",
+                     "single_direction": {"kernel": ("census_tc_kernel" if tc["left"] else "census_match_kernel<0>") +
+                                                    " (left-to-right alone, process())",
                                           "kernel_ms": round(match_ms, 4),
                                           "popc_equivalent_frac": round(single_popc / popc_peak, 4)},
                      "peak_source": "nominal dense FP4 (no measured FP4 rate); popc_equivalent: 2 POPC per cost "
@@ -610,6 +623,7 @@ def run_ours(args):
 def profile_config(args):
     """--profile <configuration>: that configuration's step twice on its own
     inputs (the sizes the bench measures), nothing else."""
+    import numpy as np
     import torch
     import ctstereo as ct
     dev = torch.device("cuda", 0)
@@ -629,9 +643,19 @@ def profile_config(args):
         m = ct.BatchStereo()
         m.configure(0, shapes, tol=1)
         step = lambda: m.process(pairs)
+    elif wl == "net_gradient":
+        import confnet_train as T
+        n = 8192
+        g = torch.Generator(device=dev).manual_seed(SEED)
+        x = torch.randint(0, 197, (n, 128), dtype=torch.uint8, device=dev, generator=g)
+        y = torch.randint(0, 2, (n,), dtype=torch.uint8, device=dev, generator=g)
+        m = ct.ConfNet()
+        m.configure(0, n)
+        m.set_params(T.load_weights())
+        step = lambda: m.loss_grad(x, y)
     else:
         W, H, D, kind = {"sad640": (640, 480, 64, 1), "ncc1080": (1920, 1080, 128, 2), "aw1440": (2560, 1440, 256, 3),
-                         "compat_ncc1080": (1920, 1080, 128, 2), "ncc1080_cuda_cores": (1920, 1080, 128, 2)}[wl]
+                         "ncc1080g": (1920, 1080, 128, 2), "compat_ncc1080": (1920, 1080, 128, 2), "ncc1080_cuda_cores": (1920, 1080, 128, 2)}[wl]
         L, R, _, _ = ct.synth_pair(kind, SEED, W, H, D - 1)
         dL, dR = up(L), up(R)
         if wl == "sad640":
@@ -646,6 +670,18 @@ def profile_config(args):
             out = ct.alloc_image(H, W, torch.uint8, dev)
             score = ct.alloc_image(H, W, torch.float32, dev)
             step = lambda: m.process(out, dL, dR, score=score)
+        elif wl == "ncc1080g":
+            def down4(img):
+                return up(np.round(img.reshape(H // 4, 4, W // 4, 4).mean(axis=(1, 3))).astype(np.uint8))
+            lc, rc, coarse = down4(L), down4(R), ct.alloc_image(H // 4, W // 4, torch.uint8, dev)
+            mc, m = ct.BlockMatcherCensus(), ct.BlockMatcherNCC()
+            mc.configure(0, W // 4, H // 4, D // 4)
+            m.configure(0, W, H, D, radius=5)
+            out, score = ct.alloc_image(H, W, torch.uint8, dev), ct.alloc_image(H, W, torch.float32, dev)
+
+            def step():
+                mc.process_lr(lc, rc, disp_checked=coarse, tol=1)
+                m.process(out, dL, dR, score=score, disp_init=coarse)
         elif wl == "aw1440":
             m = ct.BlockMatcherAW()
             m.configure(0, W, H, D)
@@ -837,7 +873,7 @@ def workload_line(wl, args, ct, dev, stream, flush_buf, world, rank, local, rate
             dr, _ = oracle.match_census(L, R, D, 2, False)
             oracle.crosscheck(dl, dr, 1, True)
             return 2 * L.shape[0] * L.shape[1] * D / (time.perf_counter() - t0) / 1e6, f"pair 0 alone ({L.shape[1]}x{L.shape[0]}, D={D})"
-        launches = 2
+        launches = 3  # census, matching, cross-check
     elif wl == "mip1080":
         # disparity mip-maps of a 1920x1080 U16 code map: the ground truth of
         # the seeded census pair (codes d + 1, occluded pixels CannotEvaluate),

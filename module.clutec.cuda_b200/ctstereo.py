@@ -402,6 +402,13 @@ class BlockMatcherCensus(_Driver):
                                                 _img_ref(right), _stream(stream)))
 
 
+def tuning_on_tensor_cores(tuning) -> dict:
+    """Which passes of a BlockMatcherCensus.tuning() run on the tensor cores: of the
+    left view alone, the right view alone, both."""
+    k = tuning["strip_height"] // CT_TUNING_TC_LEFT
+    return {"left": bool(k & 1), "right": bool(k & 2), "both": bool(k & 4)}
+
+
 class CurveVolume:
     """Device cost-curve volume (ct_curves): rows (y, g) of 32-bit words, word
     x + 2 of row (y, g) = codes of disparities 4g .. 4g + 3 at column x."""
