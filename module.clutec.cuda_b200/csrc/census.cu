@@ -334,16 +334,22 @@ int census_match_pass(BmCensusHandle* h, int dir, const ct_image* disp, cudaStre
                     : census_match_pass_maps(h, 1, disp, h->tm_rb, h->tm_lm, s, curves);
 }
 
-// Where the tensor-core pass (census_tc.cuh) is the faster one, over whole calls
-// of 160x96 .. 2560x1440 pixels. It takes about as long for few disparities as
-// for 113 (128 left pixels a tile whatever the band), so the CUDA-core pass
-// wins below 48 on images that fill the GPU: at 1920x1080 checked maps take
-// 124 us against 111 (CUDA cores) for D = 32, 124 / 124 for 48, 123 / 136 for
-// 64, 138 / 263 for 128, 255 / 506 for 256. Small images are latency-bound and
-// its single launch without a merge wins at every D (640x480: 35 / 37 us at D
-// = 32, 37 / 68 at 128; 160x96: 21 / 29 at 64). The right view alone needs the
-// key plane set and read: from 65 disparities (1920x1080: 111 / 114 us at 64,
-// 113 / 194 at 96).
+// Where the tensor-core pass (census_tc.cuh) runs, by whole calls of 160x96 ..
+// 2560x1440 pixels on either kernel. It takes about as long for few disparities
+// as for 113 (128 left pixels a tile whatever the band), so the CUDA-core pass
+// wins for few on images that fill the GPU. At 1920x1080 (us, tensor / CUDA
+// cores):
+//   D           4         16        32        40        48        64        128
+//   left     78 / 74   82 / 74   84 / 86   84 / 99   88 / 99   95 / 115  121 / 223
+//   checked 109 / 101 115 / 101 116 / 115 115 / 126 116 / 127 128 / 139  144 / 266
+// Small images are latency-bound, and its single launch without a merge wins at
+// every D (left and checked: 160x96 22 / 23 and 26 / 28 at D = 4, 17 / 23 and 23
+// / 31 at 64; 640x480 23 / 26 and 33 / 37 at D = 4, 27 / 33 and 37 / 44 at 64).
+// Between the two lines both kernels take turns: at D = 4 .. 40 1024x768 takes 51
+// .. 54 us checked against 58 .. 68, 1280x720 58 .. 61 against 57 .. 66; the
+// lines leave these to the CUDA cores. The right view alone needs the key plane
+// set and read: 640x480 35 / 33 us at D = 64, 1920x1080 109 / 113 at 64 and 115
+// / 193 at 96, hence from 65 disparities.
 bool tc_faster(int W, int H, int D, bool left) {
     if (!left) return D > 64;
     return D >= 48 || (long)W * H <= 400000;

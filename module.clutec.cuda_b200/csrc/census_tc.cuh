@@ -46,7 +46,7 @@
 // 120 cycles = 2400 cycles; the left view alone runs at that rate (2400 cycles
 // a row traced), both views at about 2900, by the maxima's instructions (3830 a
 // tile and row, 2.6 of 4 issued per cycle). Whole calls there: left view 121 us
-// (224 on the CUDA cores), both views and check 138 us (263).
+// (223 on the CUDA cores), both views and check 144 us (266).
 //
 #pragma once
 

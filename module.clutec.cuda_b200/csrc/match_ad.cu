@@ -576,10 +576,11 @@ int set_attr() {
 // Disparities per warp: 4 (16 warps per CTA) for the adaptive windows and
 // the SAD windows from 7x7 up, which are bound by instruction latency at one
 // CTA per SM; 8 for the smaller SAD windows, where loading each base pixel
-// for 8 disparities saves more than the extra warps hide (measured when the
-// costs were formed two at a time: AW 2560x1440 1.162 -> 1.025 ms and SAD 9x9
-// 640x480 0.0266 -> 0.0245 ms with 4; SAD 5x5 1920x1080 0.1833 ms with 8
-// against 0.1933 with 4).
+// for 8 disparities saves more than the extra warps hide. Whole calls, 4 / 8
+// disparities, us: 1920x1080 D = 128 AW 255 / 299, SAD 9x9 177 / 178, 7x7 175 /
+// 175, 5x5 181 / 166, 3x3 164 / 158; D = 40 AW 143 / 195, 9x9 and 7x7 62 / 68,
+// 5x5 68 / 62, 3x3 58 / 60; 640x480 D = 64 AW 36 / 42, 9x9 17.7 / 20.9, 7x7 16.9
+// / 19.2, 5x5 16.8 / 18.8, 3x3 17.7 / 16.7.
 template <int R, bool AW>
 constexpr int dpw_for() { return (AW || R >= 3) ? 4 : 8; }
 
