@@ -248,6 +248,11 @@ class ClockSampler:
                 "reasons": reasons, "samples": len(rows)}
 
 
+def launch_shape(ct, tuning):
+    """The CUDA-core kernel's shape of a tuning, without the kernels' flags."""
+    return {**tuning, "strip_height": tuning["strip_height"] % ct.CT_TUNING_TC_LEFT}
+
+
 def traffic_from_profile(tensor_cores):
     """DRAM bytes per launch of the headline's matching pass (on the tensor or
     the CUDA cores) from the committed ncu summary."""
@@ -560,7 +565,7 @@ def run_ours(args):
         "metric": METRIC, "value": round(value, 1), "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(ms, 4), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "u8 pixels / u64 census / int costs", "data": "synthetic (seeded generator)",
-        "config": census_config(), "parallelism": f"replicas x{world}", "launch_shape": {**tuning, "strip_height": tuning["strip_height"] % ct.CT_TUNING_TC_LEFT},
+        "config": census_config(), "parallelism": f"replicas x{world}", "launch_shape": launch_shape(ct, tuning),
         "on_tensor_cores": ct.tuning_on_tensor_cores(tuning),
         "e2e": {"value": round(e2e_stream, 1), "unit": UNIT, "ms_per_step": round(stream_ms, 4),
                 "h2d_bytes_per_step": 2 * W_ * H_, "d2h_bytes_per_step": W_ * H_,
@@ -655,7 +660,8 @@ def profile_config(args):
         step = lambda: m.loss_grad(x, y)
     else:
         W, H, D, kind = {"sad640": (640, 480, 64, 1), "ncc1080": (1920, 1080, 128, 2), "aw1440": (2560, 1440, 256, 3),
-                         "ncc1080g": (1920, 1080, 128, 2), "compat_ncc1080": (1920, 1080, 128, 2), "ncc1080_cuda_cores": (1920, 1080, 128, 2)}[wl]
+                         "ncc1080g": (1920, 1080, 128, 2), "compat_ncc1080": (1920, 1080, 128, 2),
+                         "ncc1080_cuda_cores": (1920, 1080, 128, 2)}[wl]
         L, R, _, _ = ct.synth_pair(kind, SEED, W, H, D - 1)
         dL, dR = up(L), up(R)
         if wl == "sad640":
@@ -1168,7 +1174,7 @@ def run_confnet(args):
         "ms_per_step": c["learned_ms"], "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
         "dtype": "u8 codes / bf16 weights / fp32 accumulate", "data": "synthetic (seeded generator kind 1)",
         "config": {"workload": "confnet_1920x1080_d128", "width": W_, "height": H_, "D": D_, "seed": SEED,
-                   "l2": "flushed before every timed step (256 MiB memset)", "launch_shape": {**tuning, "strip_height": tuning["strip_height"] % ct.CT_TUNING_TC_LEFT}},
+                   "l2": "flushed before every timed step (256 MiB memset)", "launch_shape": launch_shape(ct, tuning)},
         "e2e": {"value": round(1e3 / c["learned_e2e_ms"], 1), "unit": "frames/s", "ms_per_step": c["learned_e2e_ms"],
                 "h2d_bytes_per_step": 2 * W_ * H_, "d2h_bytes_per_step": W_ * H_},
         "plain_lr_pipeline": {"value": round(1e3 / c["plain_ms"], 1), "e2e": round(1e3 / c["plain_e2e_ms"], 1),

@@ -278,7 +278,8 @@ __device__ __forceinline__ float halve(float lo, float hi, bool upper, int mask)
 // the band stay below 0 and bid for nothing. (Holding back the keys as well cost
 // 1.6% of a batch.)
 constexpr int kRowBars = 8;
-static_assert(kRowBars >= kSlots && 5 + kRowBars <= 16, "staged rows come round to a barrier after the MMA warp has joined it");
+static_assert(kRowBars >= kSlots && 5 + kRowBars <= 16,
+              "staged rows come round to a barrier after the MMA warp has joined it");
 template <int ID, int N>
 __device__ __forceinline__ void bar_arrive() {
     asm volatile("barrier.cta.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
